@@ -147,11 +147,13 @@ size_t bucket_scan_words(uint32_t len);
 uint32_t bucket_long_capacity(uint32_t n);
 void launch_sorted_weights(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, uint32_t n,
                            double *wS);
-void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *start, uint32_t ncells, double *W);
+// upTo: the running weight at each particle, NULL to leave it out
+void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *start, uint32_t n, uint32_t nRuns,
+                           double *W, double *upTo = nullptr);
 void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out);
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
-                      const double *W, const double *Wtot, uint32_t *pCount, double *pWeight, uint64_t *cellCount,
-                      double *eradCensus, DevStats *st);
+                      uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
+                      uint64_t *cellCount, double *eradCensus, DevStats *st);
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,
                       const uint64_t *pOffset, const Bank &out);

@@ -2204,8 +2204,96 @@ __global__ void k_sorted_weights(Ctx C, CensusBank cen, const uint32_t *idx, uin
         wS[q] = census_w(C, cen, idx[q]);
 }
 
-// weights[cell] (:136-141), summed in sorted order
-__global__ void k_comb_cell_sums(const double *wS, const uint32_t *start, uint32_t ncells, double *W) {
+// The comb's walks along a run add FP64 weights left to right, so that every sum
+// rounds as the reference's: a serial chain per run.  k_comb_cell_sums is the one
+// kernel that walks all of it, and it leaves the running weight at each particle
+// for the plan.  A warp takes `batch` neighbouring runs (up to 32 where there are
+// more runs than warps on the chip) and goes over their particles, which are
+// contiguous, in tiles: the tile is loaded coalesced into shared memory, the next
+// one on its way, and each lane walks its own run's part of it there.  So a long
+// run waits for its additions alone (8 cycles each; straight from memory it paid
+// an access to L2 per addition) and short runs are walked side by side.
+constexpr uint32_t WALK_WARPS = 8;
+constexpr uint32_t WALK_BLOCKS = 148 * 8;
+constexpr uint32_t WALK_TILE = 256;
+constexpr int WALK_E = WALK_TILE / 32;
+static inline uint32_t walk_batch(uint32_t nRuns) {
+    const uint32_t b = (nRuns + WALK_BLOCKS * WALK_WARPS - 1) / (WALK_BLOCKS * WALK_WARPS);
+    return b < 1 ? 1u : (b > 32 ? 32u : b);
+}
+// a thread per run: enough runs to fill the chip, short on average
+static inline bool walk_by_thread(uint32_t n, uint32_t nRuns) { return nRuns >= 100000u && n / nRuns < 256u; }
+static inline uint32_t walk_grid(uint32_t nRuns) {
+    const uint32_t perBlock = WALK_WARPS * walk_batch(nRuns);
+    const uint32_t g = (nRuns + perBlock - 1) / perBlock;
+    return g ? g : 1u;
+}
+// the weights of tile [t0, t0 + WALK_TILE), zero from `end` on
+__device__ __forceinline__ void walk_load(double (&v)[WALK_E], const double *wS, uint32_t t0, uint32_t end,
+                                          uint32_t lane) {
+#pragma unroll
+    for (int u = 0; u < WALK_E; ++u) {
+        const uint32_t q = t0 + 32u * u + lane;
+        v[u] = q < end ? wS[q] : 0.0;
+    }
+}
+
+// weights[cell] (:136-141), summed in sorted order, and the sums up to each particle (upTo, unless NULL)
+__global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_cell_sums(const double *wS, const uint32_t *start,
+                                                                    uint32_t nRuns, double *W, double *upTo,
+                                                                    uint32_t batch) {
+    __shared__ double stage[WALK_WARPS][WALK_TILE];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double *x = stage[wid];
+    const uint32_t c0 = (blockIdx.x * WALK_WARPS + wid) * batch, c = c0 + lane;
+    if (c0 >= nRuns) return;
+    const bool mine = lane < batch && c < nRuns;
+    const uint32_t a = mine ? start[c] : 0u, b = mine ? start[c + 1] : 0u;
+    const uint32_t first = __shfl_sync(FULL, a, 0), end = start[min(c0 + batch, nRuns)];
+    double s = 0.0, v[WALK_E];
+    walk_load(v, wS, first, end, lane);
+    for (uint32_t t0 = first; t0 < end; t0 += WALK_TILE) {
+#pragma unroll
+        for (int u = 0; u < WALK_E; ++u) x[32 * u + lane] = v[u];
+        __syncwarp();
+        walk_load(v, wS, t0 + WALK_TILE, end, lane);
+        const uint32_t q0 = max(a, t0), q1 = min(b, t0 + WALK_TILE);
+        if (q0 < q1) {
+            uint32_t i = q0 - t0;
+            const uint32_t i1 = q1 - t0;
+            for (; i + 8 <= i1; i += 8) {   // eight loads at a time, ahead of the additions
+                double w[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) w[u] = x[i + u];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    s += w[u];
+                    x[i + u] = s;
+                }
+            }
+            for (; i < i1; ++i) {
+                s += x[i];
+                x[i] = s;
+            }
+        }
+        __syncwarp();
+        if (upTo) {
+#pragma unroll
+            for (int u = 0; u < WALK_E; ++u) {
+                const uint32_t q = t0 + 32u * u + lane;
+                if (q < end) upTo[q] = x[32 * u + lane];
+            }
+        }
+        __syncwarp();
+    }
+    if (mine) W[c] = s;
+}
+
+// The same sums with a thread per run straight from memory: where there are runs
+// enough to fill the chip with a thread each and they are short, a warp's lines
+// stay in L1 while its lanes walk them, and nothing is staged (38 us against 50-99
+// us on 64^3 cells of 50 particles; 480 us against 43-80 on 100 cells of 1700).
+__global__ void k_comb_cell_sums_thread(const double *wS, const uint32_t *start, uint32_t ncells, double *W) {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) {
         double s = 0.0;
         for (uint32_t q = start[c]; q < start[c + 1]; ++q) s += wS[q];
@@ -2249,13 +2337,200 @@ __device__ __forceinline__ CombCell comb_cell_params(const Ctx &C, const CombPar
     return cc;
 }
 
+// pCount bit 31 marks a particle kept as is.
+constexpr uint32_t KEEP = 0x80000000u;
+
+// #{k >= 0 : (k + r) E < P}: the comb index a sequential walk holds once it
+// has passed weight P (the loop condition of :203-222 with cum = P).
+__device__ __forceinline__ uint64_t teeth_below(double P, double r, double E) {
+    if (!(P > 0.0)) return 0;
+    const double g = P / E - r;
+    uint64_t k = g > 0.0 ? static_cast<uint64_t>(ceil(g)) : 0;
+    while (k > 0 && (static_cast<double>(k - 1) + r) * E >= P) --k;
+    while ((static_cast<double>(k) + r) * E < P) ++k;
+    return k;
+}
+
+// teeth_below for P > 0 from a guess P * perE (perE about 1 / E), with the index
+// as a whole number in FP64: the index follows from the comparisons, not from the
+// guess, and costs neither a division nor 64-bit integer conversions.
+__device__ __forceinline__ double teeth_index(double P, double perE, double r, double E) {
+    double k = fmax(ceil(P * perE - r), 0.0);
+    while (k > 0.0 && ((k - 1.0) + r) * E >= P) k -= 1.0;
+    while ((k + r) * E < P) k += 1.0;
+    return k;
+}
+
+// s with x added n times, one after another (s >= 0, x > 0).  While the sum stays
+// in one binade each addition moves it by the same multiple d of the binade's
+// unit u, unless x lies halfway between two multiples; so a whole binade is one
+// exact product and one exact addition.
+__device__ __noinline__ double add_repeated(double s, double x, uint64_t n) {
+    while (n > 0) {
+        const double t = s + x;
+        --n;
+        const double prev = s;
+        s = t;
+        if (n < 16 || prev < x) continue;   // (also: the difference below is exact from here on)
+        const double d = t - prev, lost = fabs(x - d);
+        if (d == 0.0) break;
+        const uint64_t e = static_cast<uint64_t>(__double_as_longlong(t)) >> 52;   // biased exponent of t > 0
+        if (e < 64 || e >= 2046) continue;
+        const double bottom = __longlong_as_double(static_cast<long long>(e << 52));
+        const double halfUnit = __longlong_as_double(static_cast<long long>((e - 53) << 52));
+        if (prev < bottom || lost == halfUnit) continue;
+        const double room = (2.0 * bottom - t) / d - 2.0;   // steps that stay below the binade's end
+        if (!(room >= 1.0)) continue;
+        const uint64_t j = room < static_cast<double>(n) ? static_cast<uint64_t>(room) : n;
+        s = t + static_cast<double>(j) * d;
+        n -= j;
+    }
+    return s;
+}
+
+// the same for the few copies of a split particle
+__device__ __forceinline__ double add_copies(double s, double x, uint32_t n) {
+    if (n > 32) return add_repeated(s, x, n);
+    for (; n > 0; --n) s += x;
+    return s;
+}
+
 // Per cell (:161-226): the number of copies of each sorted particle, the weight
 // of those copies, and the cell's census radiation energy summed in output order
-// (RadiationIMC::postStep :2013-2016).  pCount bit 31 marks a particle kept as is.
-constexpr uint32_t KEEP = 0x80000000u;
-__global__ void k_comb_plan(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *W,
-                            const double *Wtot, uint32_t *pCount, double *pWeight, uint64_t *cellCount,
-                            double *eradCensus, DevStats *st) {
+// (RadiationIMC::postStep :2013-2016).  A warp takes its batch of cells one after
+// another, 32 particles at a time.  In a combed cell the comb index follows from
+// the running weight of k_comb_cell_sums at the particle alone (teeth_index), and
+// the census energy is that many times the same weight (add_repeated).  In a cell
+// that is kept or split the energy is the running weight, too, up to the first
+// particle that is split; only from there on is there a serial chain, over the
+// copies, walked from shared memory.
+__global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams P, const double *wS,
+                                                               const uint32_t *start, const double *W,
+                                                               const double *upTo, const double *Wtot,
+                                                               uint32_t *pCount, double *pWeight, uint64_t *cellCount,
+                                                               double *eradCensus, DevStats *st, uint32_t batch) {
+    __shared__ __align__(16) double stage[WALK_WARPS][32];
+    __shared__ __align__(16) uint32_t copies[WALK_WARPS][32];
+    const double tot = *Wtot;
+    if (!isfinite(tot)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
+    }
+    const bool none = tot == 0.0 || !isfinite(tot);
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double *x = stage[wid];
+    uint32_t *nx = copies[wid];
+    const uint32_t c = (blockIdx.x * WALK_WARPS + wid) * batch + lane;
+    const bool mine = lane < batch && c < C.ncells;
+    const uint32_t a = mine ? start[c] : 0u, b = mine ? start[c + 1] : 0u;
+    CombCell cc{};
+    double Wc = 0.0;
+    if (b > a && !none) {
+        Wc = W[c];
+        cc = comb_cell_params(C, P, c, b - a, Wc, tot);
+    }
+    double ecell = 0.0;   // of the lane's own cell
+    uint64_t m = 0;
+    for (unsigned todo = __ballot_sync(FULL, b > a); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const uint32_t ra = __shfl_sync(FULL, a, l), rb = __shfl_sync(FULL, b, l);
+        if (none) {
+            for (uint32_t q = ra + lane; q < rb; q += 32) pCount[q] = 0;
+            continue;
+        }
+        if (__shfl_sync(FULL, cc.mode, l) == 0) {   // keep or split
+            const double ideal = __shfl_sync(FULL, cc.w_ideal, l);
+            double e = __shfl_sync(FULL, Wc, l);
+            uint64_t made = 0;
+            bool chain = false;
+            double v = ra + lane < rb ? wS[ra + lane] : 0.0;
+            for (uint32_t base = ra; base < rb; base += 32) {
+                const uint32_t q = base + lane;
+                const double w = v;
+                v = q + 32 < rb ? wS[q + 32] : 0.0;   // ahead of the plan's weights, which take their place
+                const bool in = q < rb, split = in && w > 2 * ideal;
+                double ws = w;
+                uint64_t ns = in ? 1u : 0u;
+                const unsigned cut = __ballot_sync(FULL, split);
+                if (split) {
+                    ns = static_cast<uint64_t>(ceil(w / ideal));
+                    ws = w / static_cast<double>(ns);
+                }
+                if (in) {
+                    pCount[q] = split ? static_cast<uint32_t>(ns) : (1u | KEEP);
+                    pWeight[q] = ws;
+                }
+                made += cut ? warp_sum(ns) : min(32u, rb - base);
+                uint32_t i = 0;
+                if (!chain && cut) {   // the energy up to the first split particle is the running weight
+                    i = __ffs(cut) - 1;
+                    chain = true;
+                    e = base + i > ra ? upTo[base + i - 1] : 0.0;
+                }
+                if (chain) {
+                    x[lane] = ws;
+                    nx[lane] = static_cast<uint32_t>(ns < 0xFFFFFFFFull ? ns : 0xFFFFFFFFull);
+                    __syncwarp();
+                    for (; (i & 3u) != 0; ++i) e = add_copies(e, x[i], nx[i]);
+                    for (; i < 32; i += 4) {   // nothing is added beyond the run: no copies there
+                        const double2 d0 = *reinterpret_cast<const double2 *>(x + i);
+                        const double2 d1 = *reinterpret_cast<const double2 *>(x + i + 2);
+                        const uint4 k = *reinterpret_cast<const uint4 *>(nx + i);
+                        if ((k.x | k.y | k.z | k.w) <= 1u) {
+                            e += d0.x;
+                            e += d0.y;
+                            e += d1.x;
+                            e += d1.y;
+                        } else {
+                            e = add_copies(e, d0.x, k.x);
+                            e = add_copies(e, d0.y, k.y);
+                            e = add_copies(e, d1.x, k.z);
+                            e = add_copies(e, d1.y, k.w);
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            if (static_cast<int>(lane) == l) {
+                ecell = e;
+                m = made;
+            }
+        } else {   // comb
+            const double r = __shfl_sync(FULL, cc.r, l), newEnergy = __shfl_sync(FULL, cc.e, l);
+            const double perE = 1.0 / newEnergy;
+            double before = 0.0;   // the comb index at the particle before
+            double p = ra + lane < rb ? upTo[ra + lane] : 0.0;
+            for (uint32_t base = ra; base < rb; base += 32) {
+                const uint32_t q = base + lane;
+                const bool in = q < rb;
+                const double k = in ? teeth_index(p, perE, r, newEnergy) : 0.0;
+                p = q + 32 < rb ? upTo[q + 32] : 0.0;
+                double k0 = __shfl_up_sync(FULL, k, 1);
+                if (lane == 0) k0 = before;
+                before = __shfl_sync(FULL, k, static_cast<int>(min(32u, rb - base) - 1));
+                if (in) {
+                    pCount[q] = static_cast<uint32_t>(k - k0);
+                    pWeight[q] = newEnergy;
+                }
+            }
+            if (static_cast<int>(lane) == l) m = static_cast<uint64_t>(before);
+        }
+    }
+    if (cc.mode == 1) ecell = add_repeated(0.0, cc.e, m);
+    if (mine) {
+        cellCount[c] = m;
+        eradCensus[c] = ecell;
+    }
+    const double eOut = warp_sum(mine ? ecell : 0.0);
+    if (lane == 0 && eOut != 0.0) atomicAdd(&st->eCensusOut, eOut);
+}
+
+// The same plan with a thread per cell, for runs as k_comb_cell_sums_thread takes
+// them (347 us against 415 us on 64^3 cells of 50 particles, 18 us against 72 us on
+// 72^3 cells of which one in twenty holds a particle; 5.2 ms against 0.31 ms on 100
+// cells of 1700, 53 us against 18 us on 24^3 cells of 21).
+__global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *W,
+                                   const double *Wtot, uint32_t *pCount, double *pWeight, uint64_t *cellCount,
+                                   double *eradCensus, DevStats *st) {
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -2309,17 +2584,6 @@ __global__ void k_comb_plan(Ctx C, CombParams P, const double *wS, const uint32_
     }
     eOut = warp_sum(eOut);
     if ((threadIdx.x & 31) == 0 && eOut != 0.0) atomicAdd(&st->eCensusOut, eOut);
-}
-
-// #{k >= 0 : (k + r) E < P}: the comb index a sequential walk holds once it
-// has passed weight P (the loop condition of :203-222 with cum = P).
-__device__ __forceinline__ uint64_t teeth_below(double P, double r, double E) {
-    if (!(P > 0.0)) return 0;
-    const double g = P / E - r;
-    uint64_t k = g > 0.0 ? static_cast<uint64_t>(ceil(g)) : 0;
-    while (k > 0 && (static_cast<double>(k - 1) + r) * E >= P) --k;
-    while ((static_cast<double>(k) + r) * E < P) ++k;
-    return k;
 }
 
 // Exchange 2 of a sharded comb: every (shard, cell) run's weight and particle
@@ -3242,17 +3506,27 @@ void launch_sorted_weights(cudaStream_t s, const Ctx &C, const CensusBank &cen, 
                            double *wS) {
     if (n) k_sorted_weights<<<grid_for(n, 256, 8192), 256, 0, s>>>(C, cen, idx, n, wS);
 }
-void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *start, uint32_t ncells, double *W) {
-    k_comb_cell_sums<<<grid_for(ncells, 128, 8192), 128, 0, s>>>(wS, start, ncells, W);
+void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *start, uint32_t n, uint32_t nRuns,
+                           double *W, double *upTo) {
+    if (walk_by_thread(n, nRuns)) {   // the plan by threads needs no running weights
+        k_comb_cell_sums_thread<<<grid_for(nRuns, 128, 8192), 128, 0, s>>>(wS, start, nRuns, W);
+        return;
+    }
+    k_comb_cell_sums<<<walk_grid(nRuns), 32 * WALK_WARPS, 0, s>>>(wS, start, nRuns, W, upTo, walk_batch(nRuns));
 }
 void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out) {
     k_blocked_sum<<<1, 1024, 0, s>>>(v, n, out);
 }
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
-                      const double *W, const double *Wtot, uint32_t *pCount, double *pWeight, uint64_t *cellCount,
-                      double *eradCensus, DevStats *st) {
-    k_comb_plan<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, wS, start, W, Wtot, pCount, pWeight, cellCount,
-                                                               eradCensus, st);
+                      uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
+                      uint64_t *cellCount, double *eradCensus, DevStats *st) {
+    if (walk_by_thread(n, C.ncells)) {
+        k_comb_plan_thread<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, wS, start, W, Wtot, pCount, pWeight,
+                                                                         cellCount, eradCensus, st);
+        return;
+    }
+    k_comb_plan<<<walk_grid(C.ncells), 32 * WALK_WARPS, 0, s>>>(C, P, wS, start, W, upTo, Wtot, pCount, pWeight,
+                                                                cellCount, eradCensus, st, walk_batch(C.ncells));
 }
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,

@@ -1789,7 +1789,7 @@ static int comb_sharded(StormHandle *h) {
         }
     }
     // exchange 2: run weights and counts
-    launch_comb_cell_sums(h->stream, wS, start, static_cast<uint32_t>(R), h->shardRunW);
+    launch_comb_cell_sums(h->stream, wS, start, n, static_cast<uint32_t>(R), h->shardRunW);
     launch_shard_pack_runs(h->stream, h->shardRunW, start, static_cast<uint32_t>(R), h->xbuf);
     h->launches += 2;
     CK(cudaGetLastError());
@@ -1896,8 +1896,9 @@ int storm_cuda_phase_comb(StormHandle *h) {
     const uint64_t nRuns = static_cast<uint64_t>(N) * B;
     uint32_t *start = strat ? h->stratStart : h->combStart;
     // the key kernel's compact copy of the census weights, for the bucket sort's
-    // sorted-weight gather; the plan's output offsets take that space later
-    double *wc = reinterpret_cast<double *>(h->pOff);
+    // sorted-weight gather; then the running weights of the cells' sums, for the
+    // plan; then the plan's output offsets
+    double *wc = reinterpret_cast<double *>(h->pOff), *upTo = wc;
     if (strat) launch_strat_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, h->strat, wc);
     else launch_comb_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, wc);
     int cellBits = 0;
@@ -1927,13 +1928,13 @@ int storm_cuda_phase_comb(StormHandle *h) {
     // first start[nRuns] are particles, the rest count zero)
     auto plan_and_scan = [&]() {
         if (strat) launch_strat_sums(h->stream, wS, start, N, B, h->stratBinW, h->combW);
-        else launch_comb_cell_sums(h->stream, wS, start, N, h->combW);
+        else launch_comb_cell_sums(h->stream, wS, start, n, N, h->combW, upTo);
         launch_blocked_sum(h->stream, h->combW, N, h->combWtot);
         if (strat)
             launch_strat_plan(h->stream, h->C, P, h->strat, wS, start, h->stratBinW, h->combW, h->combWtot, h->pCount,
                               h->pWeight, h->combCount, h->A.eradCensus, h->dStats);
         else
-            launch_comb_plan(h->stream, h->C, P, wS, start, h->combW, h->combWtot, h->pCount, h->pWeight,
+            launch_comb_plan(h->stream, h->C, P, wS, start, n, h->combW, upTo, h->combWtot, h->pCount, h->pWeight,
                              h->combCount, h->A.eradCensus, h->dStats);
         uint64_t *countU64 = skeys == h->keysAlt ? h->keys : h->keysAlt;   // the sort's spare key buffer
         launch_mask_count_upto(h->stream, h->pCount, n, start + nRuns, countU64);
