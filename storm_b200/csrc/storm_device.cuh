@@ -19,8 +19,12 @@ namespace storm {
 
 // ParticleStatus (particle/ParticleStatus.hpp:8-15)
 enum : int { NO_CELL_MOVE = 0, CELL_MOVE = 1, DONE = 2, REMOVE = 3, REFLECT = 4 };
+// a scatter whose new direction (and frequency) the caller still draws (finish64)
+enum : int { SCATTER = 5, SCATTER_EFFECTIVE = 6 };
 // outcome of a segment after the manager's handling
 enum : int { OUT_CONTINUE = 0, OUT_CENSUS = 1, OUT_CUTOFF = 2, OUT_ESCAPE = 3, OUT_ERROR = -1 };
+// left by a segment of the persistent transport for its finish (finish64, finish32)
+enum : int { OUT_SCATTER = 4, OUT_REEMIT = 5 };
 // random stream tags
 enum : uint32_t { TAG_TRANSPORT = 1, TAG_CELL_EMIT = 2, TAG_FACE_EMIT = 3, TAG_COMB = 4 };
 
@@ -66,6 +70,7 @@ struct RwTables {
 // Everything a kernel needs, passed by value.
 struct Ctx {
     uint32_t nx, ny, nz, ncells;
+    uint32_t nxMagic, nyMagic;   // floor(2^32 / n) + 1 (div_small)
     const double *xe, *ye, *ze, *xc, *yc, *zc;
     double X0, X1, Y0, Y1, Z0, Z1;
     BoxFaceDev bf[6];
@@ -85,6 +90,7 @@ struct Ctx {
     double rwMinParticle, rwMinCell;
     double sourceT[6];       // source temperature of each box face [K]
     uint32_t seedLo, seedHi, step;
+    uint32_t philoxKey[20];  // the ten rounds' Philox keys of the seed (k0, k1 in turn), set with it
     // FP32-tracking form
     int32_t fp32;            // banks hold cell-local FP32 offsets and FP32 directions
     const float *hx, *hy, *hz;   // half widths per axis
@@ -97,6 +103,7 @@ struct Ctx {
     const double *sigA, *sigS, *fleck, *rwSigT;
     const uint8_t *rwElig;
     double *eint, *eradAvg;
+    double *att;             // per cell: attenuation not yet added to the two tallies (gray problems; zero between steps)
     uint32_t *segs;
     RwTables rw;
     int32_t *err;            // [0] code, [1] cell lo, [2] particle lo
@@ -182,6 +189,21 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t
     out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
 }
 
+// The same block with the step's counter words and the round keys from the context.
+__device__ __forceinline__ void philox_block(const Ctx &C, uint32_t block, uint32_t pid, uint32_t tag, uint4 &out) {
+    uint32_t c0 = block, c1 = pid, c2 = C.step, c3 = tag;
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        const uint64_t p0 = static_cast<uint64_t>(0xD2511F53u) * c0;
+        const uint64_t p1 = static_cast<uint64_t>(0xCD9E8D57u) * c2;
+        const uint32_t hi0 = static_cast<uint32_t>(p0 >> 32), lo0 = static_cast<uint32_t>(p0);
+        const uint32_t hi1 = static_cast<uint32_t>(p1 >> 32), lo1 = static_cast<uint32_t>(p1);
+        const uint32_t n0 = hi1 ^ c1 ^ C.philoxKey[2 * r], n2 = hi0 ^ c3 ^ C.philoxKey[2 * r + 1];
+        c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
+    }
+    out = make_uint4(c0, c1, c2, c3);
+}
+
 // 52-bit uniform on the open interval: (m + 0.5) * 2^-52.
 __device__ __forceinline__ double u52(uint32_t a, uint32_t b) {
     uint64_t m = (static_cast<uint64_t>(a >> 6) << 26) | static_cast<uint64_t>(b >> 6);
@@ -235,6 +257,7 @@ struct PhiloxRng {
     }
     // a draw whose value is not used
     __device__ __forceinline__ void skip() { ++draw; }
+    __device__ __forceinline__ void ready(const Ctx &, uint32_t) {}   // draws make their own blocks
     // RadiationIMC::randomUnitOpen (radiation/RadiationIMC.hpp:700-713); a no-op on
     // these uniforms, kept for the shared code path.
     __device__ __forceinline__ double open() {
@@ -269,6 +292,63 @@ struct PhiloxRng4 {
         return u23(word);
     }
     __device__ __forceinline__ void skip() {}
+    __device__ __forceinline__ void ready(const Ctx &, uint32_t) {}   // draws make their own blocks
+    __device__ __forceinline__ bool exhausted() const { return false; }
+};
+
+// The streams of the persistent transport: a stream's words go through a ring of
+// kBlocks Philox blocks per thread in shared memory, and a draw reads them there.
+// A segment calls ready(n) for the draws it can take, which makes the blocks that
+// are still missing: Philox is computed at one place per segment, for all lanes
+// that run short, where a stream that makes a block at the draw that needs it
+// computes it at each draw for the few lanes whose block ends there, and holds a
+// copy of its code at every draw.  (Larger rings filled more rarely, at a vote of
+// the lanes, take shared memory from L1, and the transports lost by it.)
+template <uint32_t kPerBlock, uint32_t kBlocks>
+struct PhiloxRing {
+    static constexpr uint32_t kWords = 4 * kBlocks, kRing = kPerBlock * kBlocks;
+    uint32_t *ring;            // [kWords][256], this thread's column
+    uint32_t pid, draw, next;  // next: the first block not yet made
+    __device__ __forceinline__ void init(const Ctx &, uint32_t *r, uint32_t p, uint32_t d) {
+        ring = r + threadIdx.x;
+        pid = p;
+        draw = d;
+        next = d / kPerBlock;
+    }
+    // n <= kRing - kPerBlock + 1 draws ahead: then the block a new one replaces has been drawn
+    __device__ __forceinline__ void ready(const Ctx &C, uint32_t n) {
+        while (kPerBlock * next < draw + n) {
+            uint4 o;
+            philox_block(C, next, pid, TAG_TRANSPORT, o);
+            uint32_t *w = ring + (next % kBlocks) * 1024u;
+            w[0] = o.x;
+            w[256] = o.y;
+            w[512] = o.z;
+            w[768] = o.w;
+            ++next;
+        }
+    }
+};
+// PhiloxRng4's stream: a 23-bit float per word
+struct PhiloxRing4 : PhiloxRing<4, 2> {
+    __device__ __forceinline__ float rawf() {
+        const float u = u23(ring[(draw % kRing) * 256u]);
+        ++draw;
+        return u;
+    }
+    __device__ __forceinline__ void skip() {}
+    __device__ __forceinline__ bool exhausted() const { return false; }
+};
+// PhiloxRng's stream: a 52-bit double per two words
+struct PhiloxRing2 : PhiloxRing<2, 4> {
+    __device__ __forceinline__ double raw() {
+        const uint32_t *w = ring + (draw % kRing) * 512u;
+        ++draw;
+        return u52(w[0], w[256]);
+    }
+    __device__ __forceinline__ void skip() { ++draw; }   // a draw whose value is not used
+    // RadiationIMC::randomUnitOpen: a no-op on these uniforms, which lie inside (0, 1)
+    __device__ __forceinline__ double open() { return raw(); }
     __device__ __forceinline__ bool exhausted() const { return false; }
 };
 
@@ -289,6 +369,7 @@ struct TapeRng {
         return fminf(fmaxf(static_cast<float>(raw()), 0x1p-24f), 0x1.fffffep-1f);
     }
     __device__ __forceinline__ void skip() { (void)raw(); }
+    __device__ __forceinline__ void ready(const Ctx &, uint32_t) {}
     __device__ __forceinline__ bool exhausted() const { return over; }
 };
 
@@ -299,11 +380,22 @@ struct PartReg {
     uint32_t cell;
 };
 
+// n / d with the remainder, for magic = floor(2^32 / d) + 1 (d >= 2): the high
+// half of n * magic is the quotient or one above it (the excess is below
+// n / 2^32), and then the remainder wraps.  A few instructions where the general
+// division takes about thirty; every refill of the transport does two.
+__device__ __forceinline__ uint32_t div_small(uint32_t n, uint32_t d, uint32_t magic, uint32_t &rem) {
+    uint32_t q = d == 1 ? n : __umulhi(n, magic);
+    rem = n - q * d;
+    if (rem >= d) {
+        --q;
+        rem += d;
+    }
+    return q;
+}
 __device__ __forceinline__ void cell_ijk(const Ctx &C, uint32_t c, uint32_t &i, uint32_t &j, uint32_t &k) {
-    i = c % C.nx;
-    uint32_t r = c / C.nx;
-    j = r % C.ny;
-    k = r / C.ny;
+    const uint32_t r = div_small(c, C.nx, C.nxMagic, i);
+    k = div_small(r, C.ny, C.nyMagic, j);
 }
 
 // STORM::fallback::abs (elementary/PointOps.hpp:71)
@@ -370,20 +462,23 @@ __device__ __forceinline__ void isotropic(RNG &rng, double c, double &vx, double
 // (Erad_time_avg_[cell]).  LocalTally sums one segment's deposits (replay).
 struct LocalTally {
     static constexpr bool kEg = false;   // no group time averages
+    static constexpr bool kRun = false;
+    __device__ __forceinline__ void leave(const struct Ctx &, uint32_t) {}
     double mat_, rad_;
     double mx_, my_, mz_;   // momentum (moving material)
-    __device__ __forceinline__ void mat(uint32_t, double v) { mat_ += v; }
-    __device__ __forceinline__ void rad(uint32_t, double v) { rad_ += v; }
+    __device__ __forceinline__ void mat(const struct Ctx &, uint32_t, double v) { mat_ += v; }
+    __device__ __forceinline__ void rad(const struct Ctx &, uint32_t, double v) { rad_ += v; }
     __device__ __forceinline__ void mom(const struct Ctx &, uint32_t, double x, double y, double z) {
         mx_ += x; my_ += y; mz_ += z;
     }
 };
-// The transport kernels' tally: every segment adds its deposits to the cell with
-// fire-and-forget atomics (RED) and counts itself for the per-cell segment
-// counters.  (Summing a run of segments in one cell in registers first costs
-// more in register spills than it saves in atomics.)
+// The tally of the bank visits and of the multigroup and moving-material
+// transports: every segment adds its deposits to the cell with fire-and-forget
+// atomics (RED) and counts itself for the per-cell segment counters.
 struct SegmentTally {
     static constexpr bool kEg = false;   // no group time averages
+    static constexpr bool kRun = false;
+    __device__ __forceinline__ void leave(const struct Ctx &, uint32_t) {}   // nothing is held back
     double *eint, *erad;
     uint32_t *segs;        // NULL: no per-cell counters
     double depSum;
@@ -391,11 +486,34 @@ struct SegmentTally {
         eint = e; erad = a; segs = sc; depSum = 0.0;
     }
     __device__ __forceinline__ void enter(uint32_t c) { if (segs) atomicAdd(segs + c, 1u); }
-    __device__ __forceinline__ void mat(uint32_t c, double v) { atomicAdd(eint + c, v); depSum += v; }
-    __device__ __forceinline__ void rad(uint32_t c, double v) { atomicAdd(erad + c, v); }
+    __device__ __forceinline__ void mat(const struct Ctx &, uint32_t c, double v) { atomicAdd(eint + c, v); depSum += v; }
+    __device__ __forceinline__ void rad(const struct Ctx &, uint32_t c, double v) { atomicAdd(erad + c, v); }
     __device__ __forceinline__ void mom(const struct Ctx &C, uint32_t c, double x, double y, double z);
 };
-// The same with the group time averages (withEgTimeAvg): every Erad_time_avg
+// The tally of the gray transports.  A gray cell has one absorption rate, so what a
+// segment's attenuation adds to the radiation tally is what it adds to the
+// material times -1 / rate: one sum serves both (C.att; k_fold_attenuation adds
+// it to the two tallies after the transport).  It is kept in a register while
+// the history stays in its cell and added once when it leaves, with the count
+// of the segments.  The two to three REDs a segment took before held the gray
+// FP32 transport back by a fifth on 64^3 cells and by 40 % on 24^3 cells, where
+// fewer addresses share them.
+struct SegmentTallyRun {
+    static constexpr bool kEg = false;
+    static constexpr bool kRun = true;
+    double run;            // attenuated energy of the stay in the present cell
+    uint32_t count;        // its segments
+    double *sum;           // this thread's other deposits of the step (shared memory)
+    __device__ __forceinline__ void begin(double *s) { run = 0.0; count = 0; sum = s; }
+    __device__ __forceinline__ void enter(uint32_t) { ++count; }
+    __device__ __forceinline__ void attenuate(double v) { run -= v; }   // v = weight * expm1(-tau)
+    __device__ __forceinline__ void leave(const struct Ctx &C, uint32_t c);
+    // what is not an attenuation at the cell's rate
+    __device__ __forceinline__ void mat(const struct Ctx &C, uint32_t c, double v);
+    __device__ __forceinline__ void rad(const struct Ctx &C, uint32_t c, double v);
+    __device__ __forceinline__ void mom(const struct Ctx &, uint32_t, double, double, double) {}   // material at rest
+};
+// SegmentTally with the group time averages (withEgTimeAvg): every Erad_time_avg
 // contribution also goes to Eg_time_avg[cell][findGroup(frequency)] with the
 // particle's lab frequency at that moment (radiation/RadiationIMC.hpp:1166-1172,
 // 1485-1491, 1802-1808).  The kernels that take it are instantiated apart, so
@@ -450,8 +568,8 @@ struct SegmentTallyFixed : SegmentTally {
     unsigned long long *fm, *fr;
     double sm, sr;
     __device__ __forceinline__ void init_fixed(const struct Ctx &C);
-    __device__ __forceinline__ void mat(uint32_t c, double v) { fixed_add(fm, c, v * sm); depSum += v; }
-    __device__ __forceinline__ void rad(uint32_t c, double v) { fixed_add(fr, c, v * sr); }
+    __device__ __forceinline__ void mat(const struct Ctx &, uint32_t c, double v) { fixed_add(fm, c, v * sm); depSum += v; }
+    __device__ __forceinline__ void rad(const struct Ctx &, uint32_t c, double v) { fixed_add(fr, c, v * sr); }
 };
 
 // ------------------------------------------------------------------ multigroup
@@ -664,6 +782,11 @@ struct PolyGeom {
     }
 };
 
+template <class TALLY>
+__device__ __forceinline__ void run_attenuate(TALLY &tal, double v) {
+    if constexpr (TALLY::kRun) tal.attenuate(v);
+}
+
 // ------------------------------------------------------------------ moving material
 __device__ __forceinline__ void SegmentTally::mom(const Ctx &C, uint32_t c, double x, double y, double z) {
     double *m = C.mom + 3 * static_cast<size_t>(c);
@@ -671,6 +794,20 @@ __device__ __forceinline__ void SegmentTally::mom(const Ctx &C, uint32_t c, doub
     atomicAdd(m + 1, y);
     atomicAdd(m + 2, z);
 }
+
+__device__ __forceinline__ void SegmentTallyRun::leave(const Ctx &C, uint32_t c) {
+    if (run != 0.0) {
+        atomicAdd(C.att + c, run);
+        run = 0.0;
+    }
+    if (C.perCellCounters) atomicAdd(C.segs + c, count);
+    count = 0;
+}
+__device__ __forceinline__ void SegmentTallyRun::mat(const Ctx &C, uint32_t c, double v) {
+    atomicAdd(C.eint + c, v);
+    *sum += v;
+}
+__device__ __forceinline__ void SegmentTallyRun::rad(const Ctx &C, uint32_t c, double v) { atomicAdd(C.eradAvg + c, v); }
 
 // computeDopplerShift (radiation/RadiationIMC.hpp:228-245): the lab-to-comoving
 // factor gamma (1 - v.u / c^2) for a particle of lab velocity u in a cell
@@ -760,6 +897,7 @@ __device__ inline int try_random_walk(const Ctx &C, PartReg &p, RNG &rng, TALLY 
     struct { double vx, vy, vz, w; } old{};   // (:1121-1122), moving material only
     if constexpr (HYDRO) { old.vx = p.vx; old.vy = p.vy; old.vz = p.vz; old.w = p.w; }
     const double fl = pgrw ? C.fleck[cell] : 0.0;
+    rng.ready(C, 4);   // the leak time, an upscatter, the direction
     double tauLeak = rw_sample_leak(C.rw, rng.open());
     double tLeak = tauLeak * Ro * Ro / Dphys;
     double tCensus = p.t;
@@ -775,15 +913,19 @@ __device__ inline int try_random_walk(const Ctx &C, PartReg &p, RNG &rng, TALLY 
     else { ev = 2; dt = tUp; }
     const double rate = pgrw ? sigmaAeff * fl * c : cp.y;   // sigma_a_eff * f * c
     double rwExp = expm1(-dt * rate);
-    if (!C.noFeedback) tal.mat(cell, -rwExp * p.w);
-    if (rate > 0.0) tal.rad(cell, p.w * rwExp * (pgrw ? (-1.0 / rate) : cp.z));
+    if constexpr (TALLY::kRun) {
+        if (rate > 0.0) tal.attenuate(p.w * rwExp);   // no absorption, no deposit
+    } else {
+        if (!C.noFeedback) tal.mat(C, cell, -rwExp * p.w);
+        if (rate > 0.0) tal.rad(C, cell, p.w * rwExp * (pgrw ? (-1.0 / rate) : cp.z));
+    }
     if constexpr (TALLY::kEg) {
         if (rate > 0.0) tal.eg(C, cell, p.w * rwExp * (pgrw ? (-1.0 / rate) : cp.z), p.nu);
     }
     p.w *= 1.0 + rwExp;
     p.t -= dt;
     if (fabs(p.w) < p.w0 * 1e-4) {
-        if (!C.noFeedback) tal.mat(cell, p.w);
+        if (!C.noFeedback) tal.mat(C, cell, p.w);
         return REMOVE;
     }
     double cosTheta = 2.0 * rng.open() - 1.0;
@@ -793,6 +935,7 @@ __device__ inline int try_random_walk(const Ctx &C, PartReg &p, RNG &rng, TALLY 
     double sphi, cphi;
     sincos(phi, &sphi, &cphi);
     double dx = sinTheta * cphi, dy = sinTheta * sphi, dz = cosTheta;
+    rng.ready(C, 4);   // the radius, the new direction, an upscatter's frequency
     double disp;
     if (ev == 0) disp = Ro;
     else {
@@ -909,6 +1052,7 @@ __device__ inline int try_ddmc(const Ctx &C, PartReg &p, RNG &rng, TALLY &tal, d
         if (cut == 0 || cut > C.groups) return -1;
         if (mg_clamp(C, p.nu) >= C.gb[cut]) return -1;
     }
+    rng.ready(C, 5);
     const double f = C.fleck[cell];
     const double eventRate = total;
     const double tEvent = -log(rng.open()) / eventRate;
@@ -918,14 +1062,14 @@ __device__ inline int try_ddmc(const Ctx &C, PartReg &p, RNG &rng, TALLY &tal, d
     const double absRate = dd.y * f * C.clight;
     const double oldWeight = p.w;
     const double expFactor = expm1(-dt * absRate);
-    if (!C.noFeedback) tal.mat(cell, -expFactor * oldWeight);
+    if (!C.noFeedback) tal.mat(C, cell, -expFactor * oldWeight);
     const double integrated = (absRate > 0.0) ? oldWeight * expFactor * (-1.0 / absRate) : oldWeight * dt;
-    tal.rad(cell, integrated);
+    tal.rad(C, cell, integrated);
     if constexpr (TALLY::kEg) tal.eg(C, cell, integrated, p.nu);
     p.w *= 1.0 + expFactor;
     p.t -= dt;
     if (fabs(p.w) < p.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, p.w);
+        if (!C.noFeedback) tal.mat(C, cell, p.w);
         return REMOVE;
     }
     if (censusEvent) return DONE;
@@ -980,6 +1124,7 @@ __device__ inline int try_ddmc_poly(const Ctx &C, PartReg &p, RNG &rng, TALLY &t
     }
     Ro = (Ro > 0.0) ? Ro : 0.0;
     if (Ro * dd.x < C.ddmcMinParticle) return -1;
+    rng.ready(C, 5);
     const double f = C.fleck[cell];
     const double eventRate = total;
     const double tEvent = -log(rng.open()) / eventRate;
@@ -989,13 +1134,13 @@ __device__ inline int try_ddmc_poly(const Ctx &C, PartReg &p, RNG &rng, TALLY &t
     const double absRate = dd.y * f * C.clight;
     const double oldWeight = p.w;
     const double expFactor = expm1(-dt * absRate);
-    if (!C.noFeedback) tal.mat(cell, -expFactor * oldWeight);
+    if (!C.noFeedback) tal.mat(C, cell, -expFactor * oldWeight);
     const double integrated = (absRate > 0.0) ? oldWeight * expFactor * (-1.0 / absRate) : oldWeight * dt;
-    tal.rad(cell, integrated);
+    tal.rad(C, cell, integrated);
     p.w *= 1.0 + expFactor;
     p.t -= dt;
     if (fabs(p.w) < p.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, p.w);
+        if (!C.noFeedback) tal.mat(C, cell, p.w);
         return REMOVE;
     }
     if (censusEvent) return DONE;
@@ -1085,7 +1230,27 @@ __device__ __forceinline__ void track_begin(const Ctx &C, Track &T) {
 // V = 2 is the convex-polyhedral form: the face search of
 // distanceToNearestFace over the cell's inward normals and face centroids as
 // written (alpha = ((faceCM - x).n) / (n.v), the first smallest positive).
-template <int V, class RNG, class TALLY>
+// LATER leaves a scatter to finish64 (status SCATTER or SCATTER_EFFECTIVE).
+
+// The end of a scatter: the isotropic direction and, in a multigroup problem,
+// the clamped or re-emitted frequency (:1826-1852).  False where the spectrum
+// cannot be sampled.
+template <bool MG, class RNG>
+__device__ __forceinline__ bool finish64(const Ctx &C, Track &T, RNG &rng, bool effective) {
+    PartReg &p = T.p;
+    isotropic(rng, C.clight, p.vx, p.vy, p.vz);
+    if (MG && C.groups >= 2) {
+        p.nu = mg_clamp(C, p.nu);
+        if (effective) {
+            p.nu = mg_thermal_energy(C, p.cell, rng.open());
+            if (p.nu < 0.0) return false;
+        }
+    }
+    T.speed = vnorm(p.vx, p.vy, p.vz);
+    return true;
+}
+
+template <int V, bool LATER = false, class RNG, class TALLY>
 __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &tal) {
     // V: 0 gray Cartesian, 1 + multigroup and DDMC, 2 polyhedral, 3 = 1 + moving material,
     // 4 = 1 without the DDMC branch, 5 = 2 with DDMC (the variants without a
@@ -1102,6 +1267,9 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
     o.errCode = 0;
     const uint32_t cell = p.cell;
     const uint32_t i = T.i, j = T.j, k = T.k;
+    // the draws a segment can take: the collision, the scatter's kind and direction;
+    // in a multigroup problem also the re-emission
+    rng.ready(C, FULL ? 5u : 4u);
     const double thr = EPSILON_FACE * T.speed;
     int face = -1;
     uint32_t next;
@@ -1127,19 +1295,21 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
         next = nb < C.ncells ? nb : OUTSIDE;
         if (next == OUTSIDE) o.ghost = nb;
     }
-    const double xl = POLY ? 0.0 : C.xe[i], xh = POLY ? 0.0 : C.xe[i + 1], yl = POLY ? 0.0 : C.ye[j],
-                 yh = POLY ? 0.0 : C.ye[j + 1], zl = POLY ? 0.0 : C.ze[k], zh = POLY ? 0.0 : C.ze[k + 1];
     if constexpr (!POLY) {
     // candidate face per axis: numerator (p_f - x) and velocity component
     double nb = 0.0, vb = 1.0;
     {
         double n;
         bool ok;
-        if (p.vx < -thr) { n = xl - p.x; ok = n < 0.0; } else if (p.vx > thr) { n = xh - p.x; ok = n > 0.0; } else ok = false;
+        // one plane per axis: the one ahead
+        n = C.xe[i + (p.vx > 0.0 ? 1 : 0)] - p.x;
+        ok = p.vx < -thr ? n < 0.0 : (p.vx > thr && n > 0.0);
         if (ok) { nb = n; vb = p.vx; face = p.vx > 0.0 ? 1 : 0; }
-        if (p.vy < -thr) { n = yl - p.y; ok = n < 0.0; } else if (p.vy > thr) { n = yh - p.y; ok = n > 0.0; } else ok = false;
+        n = C.ye[j + (p.vy > 0.0 ? 1 : 0)] - p.y;
+        ok = p.vy < -thr ? n < 0.0 : (p.vy > thr && n > 0.0);
         if (ok && (face < 0 || fabs(n) * fabs(vb) < fabs(nb) * fabs(p.vy))) { nb = n; vb = p.vy; face = p.vy > 0.0 ? 3 : 2; }
-        if (p.vz < -thr) { n = zl - p.z; ok = n < 0.0; } else if (p.vz > thr) { n = zh - p.z; ok = n > 0.0; } else ok = false;
+        n = C.ze[k + (p.vz > 0.0 ? 1 : 0)] - p.z;
+        ok = p.vz < -thr ? n < 0.0 : (p.vz > thr && n > 0.0);
         if (ok && (face < 0 || fabs(n) * fabs(vb) < fabs(nb) * fabs(p.vz))) { nb = n; vb = p.vz; face = p.vz > 0.0 ? 5 : 4; }
     }
     if (face < 0) { o.errCode = STORM_DERR_NO_FACE; return o; }
@@ -1181,7 +1351,7 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
             const PolyGeom g{&C, C.cfo[cell], C.cfo[cell + 1], C.mpx[cell], C.mpy[cell], C.mpz[cell]};
             r = try_random_walk<FULL>(C, p, rng, tal, cp, g);
         } else {
-            const CartGeom g{xl, xh, yl, yh, zl, zh, C.xc[i], C.yc[j], C.zc[k]};
+            const CartGeom g{C.xe[i], C.xe[i + 1], C.ye[j], C.ye[j + 1], C.ze[k], C.ze[k + 1], C.xc[i], C.yc[j], C.zc[k]};
             r = try_random_walk<FULL, CartGeom, RNG, TALLY, HYDRO>(C, p, rng, tal, cp, g);
         }
         if (r == -2) { o.errCode = STORM_DERR_RW_SHRINK; return o; }
@@ -1200,7 +1370,7 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
             const PolyGeom g{&C, C.cfo[cell], C.cfo[cell + 1], C.mpx[cell], C.mpy[cell], C.mpz[cell]};
             r = try_ddmc_poly(C, p, rng, tal, g, dnext);
         } else {
-            r = try_ddmc(C, p, rng, tal, xl, xh, yl, yh, zl, zh, dface, dnext);
+            r = try_ddmc(C, p, rng, tal, C.xe[i], C.xe[i + 1], C.ye[j], C.ye[j + 1], C.ze[k], C.ze[k + 1], dface, dnext);
         }
         if (r >= 0) {
             o.status = r;
@@ -1231,20 +1401,22 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
     const double e2 = expm1(tmp);
     const double e1 = HYDRO ? expm1(tmp * dop) : e2;
     double integrated = p.w * dt;
-    if (fabs(tmp2 * dt) >= 1e-12) integrated = p.w * e2 * cp.z;
+    const bool absorbs = fabs(tmp2 * dt) >= 1e-12;
+    if (absorbs) integrated = p.w * e2 * cp.z;
     p.x += p.vx * dt;
     p.y += p.vy * dt;
     p.z += p.vz * dt;
-    if (!C.noFeedback) tal.mat(cell, -e2 * p.w);
+    if (TALLY::kRun && absorbs) run_attenuate(tal, p.w * e2);
+    else if (!C.noFeedback) tal.mat(C, cell, -e2 * p.w);
     if (HYDRO && C.withHydro && !C.noFeedback) {   // (:1793-1798)
         const double a = -e1 * p.w;
         tal.mom(C, cell, a * p.vx * C.invC2, a * p.vy * C.invC2, a * p.vz * C.invC2);
     }
-    tal.rad(cell, integrated);
+    if (!(TALLY::kRun && absorbs)) tal.rad(C, cell, integrated);
     if constexpr (TALLY::kEg) tal.eg(C, cell, integrated, p.nu);
     p.w *= 1.0 + e1;
     if (fabs(p.w) < p.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, p.w);
+        if (!C.noFeedback) tal.mat(C, cell, p.w);
         o.status = REMOVE;
         return o;
     }
@@ -1254,30 +1426,26 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
         o.next = next;
         if (!POLY && next == OUTSIDE) o.ghost = C.ncells + face_index(C, i, j, k, face);
     } else if (best == 1) {
-        const double oldVx = p.vx, oldVy = p.vy, oldVz = p.vz;
-        if (FULL && C.groups >= 2) {
-            // elastic or effective scatter (:1826-1852): both re-scatter
-            // isotropically; an effective scatter re-emits from the spectrum
-            const double eventRandom = rng.open() * eventOpacity;
-            const bool effective = !(eventRandom < elastic);
-            isotropic(rng, c, p.vx, p.vy, p.vz);
-            p.nu = mg_clamp(C, HYDRO ? p.nu * dop : p.nu);
-            if (effective) {
-                p.nu = mg_thermal_energy(C, cell, rng.open());
-                if (p.nu < 0.0) { o.errCode = STORM_DERR_MG_SAMPLE; return o; }
-            }
-        } else {
-            rng.skip();   // event-type draw; both branches re-scatter isotropically
-            isotropic(rng, c, p.vx, p.vy, p.vz);
+        // elastic or effective scatter (:1826-1852): both re-scatter
+        // isotropically; an effective scatter re-emits from the spectrum
+        bool effective = false;
+        if (FULL && C.groups >= 2) effective = !(rng.open() * eventOpacity < elastic);
+        else rng.skip();   // event-type draw
+        if constexpr (LATER && !HYDRO) {
+            o.status = effective ? SCATTER_EFFECTIVE : SCATTER;
+            return o;
         }
+        const double oldVx = p.vx, oldVy = p.vy, oldVz = p.vz;
+        if (HYDRO) p.nu *= dop;   // dop = 1 for a cell at rest
+        if (!finish64<FULL>(C, T, rng, effective)) { o.errCode = STORM_DERR_MG_SAMPLE; return o; }
         if (HYDRO && C.withHydro) {   // the comoving scatter back to the lab frame (:1853-1871)
             const double weightBefore = p.w;
             p.w *= dop;
             lorentz_to_lab(C, cvel, p);
             if (C.groups >= 2) p.nu = mg_clamp(C, p.nu);
             if (!C.noFeedback) momentum_exchange(C, tal, cell, weightBefore, oldVx, oldVy, oldVz, p);
+            T.speed = vnorm(p.vx, p.vy, p.vz);
         }
-        T.speed = vnorm(p.vx, p.vy, p.vz);
         o.status = NO_CELL_MOVE;
     } else {
         o.status = DONE;
@@ -1292,14 +1460,57 @@ struct Track32 {
     float qx, qy, qz, ux, uy, uz;
     double t, w, w0;
     uint32_t cell, i, j, k;
-    // the constants of cell `cc`, kept in registers while the particle stays in it
-    uint32_t cc;
+    // the cell's constants (enter_cell32), kept in registers while the particle stays in it
     float4 cp;
     float hx, hy, hz;
     // multigroup: photon energy, and the cell's kT and sigma0 (cached with cp)
     float nu, kT, s0;
 };
 
+// the constants of the particle's cell, on a cell change along one axis without its half widths
+template <bool MG>
+__device__ __forceinline__ void enter_cell32(const Ctx &C, Track32 &T) {
+    T.cp = C.phys32[T.cell];
+    if (MG) {
+        T.kT = static_cast<float>(mg_kT(C, T.cell));
+        T.s0 = static_cast<float>(C.sig0[T.cell] / C.mgKTq[T.cell]);   // sigma0 / (kT)^q
+    }
+}
+template <bool MG, bool POLY>
+__device__ __forceinline__ void begin_cell32(const Ctx &C, Track32 &T) {
+    cell_ijk(C, T.cell, T.i, T.j, T.k);
+    if (!POLY) { T.hx = C.hx[T.i]; T.hy = C.hy[T.j]; T.hz = C.hz[T.k]; }
+    enter_cell32<MG>(C, T);
+}
+// Moves a particle across cell face `face` (GetCellFaces order) into the
+// neighbour: its cell, the coordinate along the face's axis ENTRY32 of the
+// half width from the centre, and the new cell's constants.  False where the
+// face lies on the box.  Written with selects: one load for all lanes that
+// cross, whichever way each goes.
+template <bool MG, class TALLY>
+__device__ __forceinline__ bool cross_face32(const Ctx &C, Track32 &T, TALLY &tal, int face) {
+    const int axis = face >> 1;
+    const bool hi = face & 1;
+    const uint32_t at = axis == 0 ? T.i : (axis == 1 ? T.j : T.k);
+    const uint32_t n = axis == 0 ? C.nx : (axis == 1 ? C.ny : C.nz);
+    if (hi ? at + 1 >= n : at == 0) return false;
+    tal.leave(C, T.cell);
+    const uint32_t to = hi ? at + 1 : at - 1;
+    const uint32_t stride = axis == 0 ? 1u : (axis == 1 ? C.nx : C.nx * C.ny);
+    T.cell = hi ? T.cell + stride : T.cell - stride;
+    const float h = (axis == 0 ? C.hx : (axis == 1 ? C.hy : C.hz))[to];
+    const float q = hi ? -h * ENTRY32 : h * ENTRY32;
+    if (axis == 0) { T.i = to; T.hx = h; T.qx = q; }
+    else if (axis == 1) { T.j = to; T.hy = h; T.qy = q; }
+    else { T.k = to; T.hz = h; T.qz = q; }
+    enter_cell32<MG>(C, T);
+    return true;
+}
+
+// v, negated where s is
+__device__ __forceinline__ float with_sign_of(float v, float s) {
+    return __uint_as_float(__float_as_uint(v) ^ (__float_as_uint(s) & 0x80000000u));
+}
 __device__ __forceinline__ float clampf(float v, float h) { return fminf(fmaxf(v, -h), h); }
 
 // RandomWalk::sampleLeakTime / sampleRadius (radiation/RandomWalk.hpp:81-137)
@@ -1377,6 +1588,7 @@ __device__ inline int rw_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         D = cp.z * C.rwDiffPerReach;
         sigAf = cp.y;
     }
+    rng.ready(C, 4);   // the leak time, an upscatter, the direction
     const float tauLeak = rw_sample_leak32(C.rw, rng.rawf());
     const double tLeak = static_cast<double>(tauLeak * (Ro * Ro) / D);
     double tUp = DBL_MAX;
@@ -1391,16 +1603,20 @@ __device__ inline int rw_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
     else { ev = 2; dt = tUp; }
     const float tau = sigAf * static_cast<float>(dt * C.clight);
     const double e1 = static_cast<double>(expm1f(-tau));
-    if (!C.noFeedback) tal.mat(cell, -e1 * T.w);
-    if (sigAf > 0.0f) {
+    if constexpr (TALLY::kRun) {
+        if (sigAf > 0.0f) tal.attenuate(T.w * e1);
+    } else {
+        if (!C.noFeedback) tal.mat(C, cell, -e1 * T.w);
+    }
+    if (!TALLY::kRun && sigAf > 0.0f) {
         const double invRate = MG ? -1.0 / (static_cast<double>(sigAf) * C.clight) : static_cast<double>(cp.w);
-        tal.rad(cell, T.w * e1 * invRate);
+        tal.rad(C, cell, T.w * e1 * invRate);
         if constexpr (TALLY::kEg) tal.eg32(C, cell, T.w * e1 * invRate, T.nu);
     }
     T.w *= 1.0 + e1;
     T.t -= dt;
     if (fabs(T.w) < T.w0 * 1e-4) {
-        if (!C.noFeedback) tal.mat(cell, T.w);
+        if (!C.noFeedback) tal.mat(C, cell, T.w);
         return OUT_CUTOFF;
     }
     const float cosT = 2.0f * rng.rawf() - 1.0f;
@@ -1408,6 +1624,7 @@ __device__ inline int rw_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
     float sphi, cphi;
     __sincosf(6.2831853f * rng.rawf(), &sphi, &cphi);
     const float dx = sinT * cphi, dy = sinT * sphi, dz = cosT;
+    rng.ready(C, MG ? 4 : 3);   // the radius, the new direction, a pending upscatter's frequency
     float disp = Ro;
     if (ev != 0) {
         const float tauPos = static_cast<float>(dt) * D / (Ro * Ro);
@@ -1434,7 +1651,7 @@ __device__ inline int rw_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         const uint32_t cutoff = C.pgrwCut[cell];
         const double *cdf = C.mgCdf + static_cast<size_t>(cell) * (C.groups + 1);
         const double cdfAtCutoff = cdf[cutoff], cdfTotal = cdf[C.groups];
-        if (cdfTotal > cdfAtCutoff)   // sampled at the start of the next segment (segment32)
+        if (cdfTotal > cdfAtCutoff)   // sampled by finish32
             T.nu = -1.0f - static_cast<float>(cdfAtCutoff / cdfTotal);
         else
             T.nu = static_cast<float>(mg_clamp(C, nextafter(C.gb[cutoff], DBL_MAX)));
@@ -1449,22 +1666,23 @@ __device__ inline int rw_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
 // the neighbour at the centre of the shared face (ENTRY32 inside it) with a
 // cosine-law direction about the face normal.  The caller has checked the
 // particle's distance to the faces against the cell's DDMC depth.
-template <class RNG, class TALLY>
+template <bool MG, class RNG, class TALLY>
 __device__ inline int ddmc_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, const float4 &da) {
     const uint32_t cell = T.cell;
+    rng.ready(C, 4);
     const double tEvent = static_cast<double>(-__logf(rng.rawf()) * da.y);
     const bool census = T.t <= tEvent;
     const double dt = census ? T.t : tEvent;
     const float tau = da.z * static_cast<float>(dt);
     const double e1 = static_cast<double>(expm1f(-tau));
-    if (!C.noFeedback) tal.mat(cell, -e1 * T.w);
-    tal.rad(cell, da.z > 0.0f ? T.w * e1 * (-1.0 / static_cast<double>(da.z)) : T.w * dt);
+    if (!C.noFeedback) tal.mat(C, cell, -e1 * T.w);
+    tal.rad(C, cell, da.z > 0.0f ? T.w * e1 * (-1.0 / static_cast<double>(da.z)) : T.w * dt);
     if constexpr (TALLY::kEg)
         tal.eg32(C, cell, da.z > 0.0f ? T.w * e1 * (-1.0 / static_cast<double>(da.z)) : T.w * dt, T.nu);
     T.w *= 1.0 + e1;
     T.t -= dt;
     if (fabs(T.w) < T.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, T.w);
+        if (!C.noFeedback) tal.mat(C, cell, T.w);
         return OUT_CUTOFF;
     }
     if (census) return OUT_CENSUS;
@@ -1484,14 +1702,7 @@ __device__ inline int ddmc_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal
     float sp, cph;
     __sincosf(phi, &sp, &cph);
     const float sg = (s & 1) ? 1.0f : -1.0f;
-    switch (s) {
-    case 0: --T.i; T.cell -= 1; T.qx = C.hx[T.i] * ENTRY32; break;
-    case 1: ++T.i; T.cell += 1; T.qx = -C.hx[T.i] * ENTRY32; break;
-    case 2: --T.j; T.cell -= C.nx; T.qy = C.hy[T.j] * ENTRY32; break;
-    case 3: ++T.j; T.cell += C.nx; T.qy = -C.hy[T.j] * ENTRY32; break;
-    case 4: --T.k; T.cell -= C.nx * C.ny; T.qz = C.hz[T.k] * ENTRY32; break;
-    default: ++T.k; T.cell += C.nx * C.ny; T.qz = -C.hz[T.k] * ENTRY32; break;
-    }
+    cross_face32<MG>(C, T, tal, s);   // a face with a leak rate has a neighbour
     const int axis = s >> 1;
     if (axis == 0) { T.qy = 0.0f; T.qz = 0.0f; T.ux = sg * mu; T.uy = st * cph; T.uz = st * sp; }
     else if (axis == 1) { T.qz = 0.0f; T.qx = 0.0f; T.uy = sg * mu; T.uz = st * cph; T.ux = st * sp; }
@@ -1508,17 +1719,18 @@ __device__ inline int ddmc_jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal
 template <class RNG, class TALLY>
 __device__ inline int ddmc_jump32_poly(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, const float4 &da) {
     const uint32_t cell = T.cell;
+    rng.ready(C, 4);
     const double tEvent = static_cast<double>(-__logf(rng.rawf()) * da.y);
     const bool census = T.t <= tEvent;
     const double dt = census ? T.t : tEvent;
     const float tau = da.z * static_cast<float>(dt);
     const double e1 = static_cast<double>(expm1f(-tau));
-    if (!C.noFeedback) tal.mat(cell, -e1 * T.w);
-    tal.rad(cell, da.z > 0.0f ? T.w * e1 * (-1.0 / static_cast<double>(da.z)) : T.w * dt);
+    if (!C.noFeedback) tal.mat(C, cell, -e1 * T.w);
+    tal.rad(C, cell, da.z > 0.0f ? T.w * e1 * (-1.0 / static_cast<double>(da.z)) : T.w * dt);
     T.w *= 1.0 + e1;
     T.t -= dt;
     if (fabs(T.w) < T.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, T.w);
+        if (!C.noFeedback) tal.mat(C, cell, T.w);
         return OUT_CUTOFF;
     }
     if (census) return OUT_CENSUS;
@@ -1556,8 +1768,10 @@ __device__ inline int ddmc_jump32_poly(const Ctx &C, Track32 &T, RNG &rng, TALLY
     T.qx = static_cast<float>(fcm.x - C.mpx[nb]) * ENTRY32;
     T.qy = static_cast<float>(fcm.y - C.mpy[nb]) * ENTRY32;
     T.qz = static_cast<float>(fcm.z - C.mpz[nb]) * ENTRY32;
+    tal.leave(C, cell);
     T.cell = nb;
     T.i = nb;
+    enter_cell32<false>(C, T);
     return OUT_CONTINUE;
 }
 
@@ -1611,31 +1825,41 @@ __device__ __forceinline__ float mg_absorption32(const Ctx &C, const Track32 &T,
 // new mesh point and is nudged 2^-21 of it toward that point.
 // DDMC = false compiles the DDMC branch out (problems without withDDMC): a
 // smaller kernel for the instruction cache.
-template <bool MG, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
+// LATER leaves a scatter (OUT_SCATTER) to finish32; a re-emission that a segment
+// leaves pending (T.nu < 0) always is.
+
+// What a segment leaves: a scatter's direction, and the re-emission from the
+// cell's spectrum that an effective scatter, or a PGRW upscatter that draws above
+// the cutoff's cumulative fraction lo, left pending as nu = -(1 + lo), in the
+// order of their draws.  False where the spectrum cannot be sampled.
+template <bool MG, class RNG>
+__device__ __forceinline__ bool finish32(const Ctx &C, Track32 &T, RNG &rng, bool scatter) {
+    if (scatter) {
+        const float theta = 6.2831853f * rng.rawf();
+        const float cosT = 2.0f * rng.rawf() - 1.0f;
+        const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
+        float st, ct;
+        __sincosf(theta, &st, &ct);
+        T.ux = sinT * ct; T.uy = sinT * st; T.uz = cosT;
+    }
+    if (MG && T.nu < 0.0f) {
+        const double lo = static_cast<double>(-T.nu - 1.0f);
+        const double nu = mg_thermal_energy(C, T.cell, lo + static_cast<double>(rng.rawf()) * (1.0 - lo));
+        if (nu < 0.0) return false;
+        T.nu = static_cast<float>(nu);
+    }
+    return true;
+}
+
+template <bool MG, bool LATER, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
 __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, int &usedRW, int &err) {
     const uint32_t cell = T.cell;
-    if (T.cc != cell) {   // entered another cell: load its constants once
-        T.cp = C.phys32[cell];
-        if (!POLY) { T.hx = C.hx[T.i]; T.hy = C.hy[T.j]; T.hz = C.hz[T.k]; }
-        T.cc = cell;
-        if (MG) {
-            T.kT = static_cast<float>(mg_kT(C, cell));
-            T.s0 = static_cast<float>(C.sig0[cell] / C.mgKTq[cell]);   // sigma0 / (kT)^q
-        }
-    }
+    // the draws a segment can take: the collision and the scatter's two; in a
+    // multigroup problem also a pending re-emission and the scatter's kind
+    rng.ready(C, MG ? 5u : 3u);
     const float hx = T.hx, hy = T.hy, hz = T.hz;
     const float4 cp = T.cp;
     if (MG) {
-        // A re-emission from the cell's spectrum that the previous segment
-        // (an effective scatter, or a PGRW upscatter that draws above the
-        // cutoff's cumulative fraction lo) left pending as nu = -(1 + lo): it
-        // is sampled here, so that the kernel holds one copy of the sampler.
-        if (T.nu < 0.0f) {
-            const double lo = static_cast<double>(-T.nu - 1.0f);
-            const double nu = mg_thermal_energy(C, cell, lo + static_cast<double>(rng.rawf()) * (1.0 - lo));
-            if (nu < 0.0) { err = STORM_DERR_MG_SAMPLE; return OUT_ERROR; }
-            T.nu = static_cast<float>(nu);
-        }
         T.nu = fminf(fmaxf(T.nu, C.gb32[0]), C.gb32[C.groups]);   // clampFrequencyToBounds
     }
 
@@ -1663,7 +1887,7 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         const float4 da = C.ddmc32[3 * static_cast<size_t>(cell)];   // depth reach, 1/total, sigma_A f c, nu bound
         if (Ro >= da.x && Ro > 0.0f && (!MG || T.nu < da.w)) {
             if constexpr (POLY) return ddmc_jump32_poly(C, T, rng, tal, da);
-            else return ddmc_jump32(C, T, rng, tal, da);
+            else return ddmc_jump32<MG>(C, T, rng, tal, da);
         }
     }
     // gray: the cell constants; multigroup: the opacity at the particle's frequency
@@ -1700,15 +1924,18 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         if (face < 0) { err = STORM_DERR_NO_FACE; return OUT_ERROR; }
         sF = bestS;
     } else {
+    // h - sign(u) q along each axis.  An axis with u = 0 never wins: it enters as
+    // distance 1 at speed 0 if it is the first, and loses the comparison otherwise.
     const float ax = fabsf(T.ux), ay = fabsf(T.uy), az = fabsf(T.uz);
-    const float nxp = ax > 0.0f ? fmaxf(hx - (T.ux > 0.0f ? T.qx : -T.qx), 0.0f) : 1.0f;
-    const float nyp = ay > 0.0f ? fmaxf(hy - (T.uy > 0.0f ? T.qy : -T.qy), 0.0f) : 1.0f;
-    const float nzp = az > 0.0f ? fmaxf(hz - (T.uz > 0.0f ? T.qz : -T.qz), 0.0f) : 1.0f;
-    float bn = nxp, bd = ax;
-    face = ax > 0.0f ? (T.ux > 0.0f ? 1 : 0) : -1;
-    if (ay > 0.0f && (face < 0 || nyp * bd < bn * ay)) { bn = nyp; bd = ay; face = T.uy > 0.0f ? 3 : 2; }
-    if (az > 0.0f && (face < 0 || nzp * bd < bn * az)) { bn = nzp; bd = az; face = T.uz > 0.0f ? 5 : 4; }
-    if (face < 0) { err = STORM_DERR_NO_FACE; return OUT_ERROR; }
+    const float nxp = fmaxf(hx - with_sign_of(T.qx, T.ux), 0.0f);
+    const float nyp = fmaxf(hy - with_sign_of(T.qy, T.uy), 0.0f);
+    const float nzp = fmaxf(hz - with_sign_of(T.qz, T.uz), 0.0f);
+    float bn = ax > 0.0f ? nxp : 1.0f, bd = ax, bu = T.ux;
+    int axis = 0;
+    if (nyp * bd < bn * ay) { bn = nyp; bd = ay; bu = T.uy; axis = 2; }
+    if (nzp * bd < bn * az) { bn = nzp; bd = az; bu = T.uz; axis = 4; }
+    if (!(bd > 0.0f)) { err = STORM_DERR_NO_FACE; return OUT_ERROR; }
+    face = axis + (bu > 0.0f ? 1 : 0);
     sF = __fdividef(bn, bd);
     }
     const double c = C.clight;
@@ -1723,8 +1950,9 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
     T.t -= dt;
     const float tau = sigAf * ds;
     const double e1 = static_cast<double>(expm1f(-tau));
+    const bool absorbs = tau >= 1e-12f;
     double integrated = T.w * dt;
-    if (tau >= 1e-12f) integrated = T.w * e1 * invRate;
+    if (absorbs) integrated = T.w * e1 * invRate;
     if constexpr (POLY) {
         T.qx = fmaf(T.ux, ds, T.qx);
         T.qy = fmaf(T.uy, ds, T.qy);
@@ -1734,27 +1962,25 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         T.qy = clampf(fmaf(T.uy, ds, T.qy), hy);
         T.qz = clampf(fmaf(T.uz, ds, T.qz), hz);
     }
-    if (!C.noFeedback) tal.mat(cell, -e1 * T.w);
-    tal.rad(cell, integrated);
+    if (TALLY::kRun && absorbs) {
+        run_attenuate(tal, T.w * e1);
+    } else {
+        if (!C.noFeedback) tal.mat(C, cell, -e1 * T.w);
+        tal.rad(C, cell, integrated);
+    }
     if constexpr (TALLY::kEg) tal.eg32(C, cell, integrated, T.nu);
     T.w *= 1.0 + e1;
     if (fabs(T.w) < T.w0 * 1e-3) {
-        if (!C.noFeedback) tal.mat(cell, T.w);
+        if (!C.noFeedback) tal.mat(C, cell, T.w);
         return OUT_CUTOFF;
     }
     if (best == 2) return OUT_CENSUS;
     if (best == 1) {
-        bool effective = false;
-        if (MG) effective = !(rng.rawf() * sigE < elastic);   // elastic or effective scatter
+        // elastic or effective scatter; an effective one re-emits from the cell's spectrum
+        if (MG && !(rng.rawf() * sigE < elastic)) T.nu = -1.0f;
         else rng.skip();   // the event-type draw (a no-op on the FP32 form's own stream)
-        const float theta = 6.2831853f * rng.rawf();
-        const float cosT = 2.0f * rng.rawf() - 1.0f;
-        const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
-        float st, ct;
-        __sincosf(theta, &st, &ct);
-        T.ux = sinT * ct; T.uy = sinT * st; T.uz = cosT;
-        if (MG && effective) T.nu = -1.0f;   // re-emission from the cell's spectrum, at the next segment's start
-        return OUT_CONTINUE;
+        if constexpr (LATER) return OUT_SCATTER;
+        return finish32<MG>(C, T, rng, true) ? OUT_CONTINUE : OUT_ERROR;
     }
     // face crossing
     if constexpr (POLY) {
@@ -1768,8 +1994,10 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
             T.qx = (T.qx + dx) * ENTRY32;
             T.qy = (T.qy + dy) * ENTRY32;
             T.qz = (T.qz + dz) * ENTRY32;
+            tal.leave(C, cell);
             T.cell = nb;
             T.i = nb;
+            enter_cell32<MG>(C, T);
             return OUT_CONTINUE;
         }
         // a box face: its axis and side from the inward normal
@@ -1787,33 +2015,14 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         return OUT_CONTINUE;
     }
     const int axis = face >> 1, hi = face & 1;
-    bool inside;
-    switch (face) {
-    case 0: inside = T.i > 0; break;
-    case 1: inside = T.i + 1 < C.nx; break;
-    case 2: inside = T.j > 0; break;
-    case 3: inside = T.j + 1 < C.ny; break;
-    case 4: inside = T.k > 0; break;
-    default: inside = T.k + 1 < C.nz; break;
-    }
-    if (inside) {
-        // The serial manager nudges a particle that changed cells 1e-8 of the
-        // way to the new cell's centre (MonteCarloManagerSerial.hpp:323-327),
-        // which an FP32 offset cannot hold.  The particle enters ENTRY32 of
-        // the half width from the centre instead: at least 4 ulps inside the
-        // face, so a cell whose mean free path is below the offset's
-        // resolution still sees a nonzero distance to the face (Random Walk
-        // eligible) rather than a particle pinned to the face.
-        switch (face) {
-        case 0: --T.i; T.cell -= 1; T.qx = C.hx[T.i] * ENTRY32; break;
-        case 1: ++T.i; T.cell += 1; T.qx = -C.hx[T.i] * ENTRY32; break;
-        case 2: --T.j; T.cell -= C.nx; T.qy = C.hy[T.j] * ENTRY32; break;
-        case 3: ++T.j; T.cell += C.nx; T.qy = -C.hy[T.j] * ENTRY32; break;
-        case 4: --T.k; T.cell -= C.nx * C.ny; T.qz = C.hz[T.k] * ENTRY32; break;
-        default: ++T.k; T.cell += C.nx * C.ny; T.qz = -C.hz[T.k] * ENTRY32; break;
-        }
-        return OUT_CONTINUE;
-    }
+    // The serial manager nudges a particle that changed cells 1e-8 of the
+    // way to the new cell's centre (MonteCarloManagerSerial.hpp:323-327),
+    // which an FP32 offset cannot hold.  The particle enters ENTRY32 of
+    // the half width from the centre instead: at least 4 ulps inside the
+    // face, so a cell whose mean free path is below the offset's
+    // resolution still sees a nonzero distance to the face (Random Walk
+    // eligible) rather than a particle pinned to the face.
+    if (cross_face32<MG>(C, T, tal, face)) return OUT_CONTINUE;
     // the box face this cell face lies on (GetBoxFaces order matches the side order)
     if (C.escapeNoCheck || C.bf[face].action == STORM_FACE_ESCAPE) return OUT_ESCAPE;
     const float sgn = hi ? 1.0f : -1.0f;
@@ -1901,6 +2110,8 @@ __device__ __forceinline__ int manager_handle(const Ctx &C, Track &T, const Phys
     }
     if (o.status == REMOVE) return OUT_CUTOFF;
     if (o.status == DONE) return OUT_CENSUS;
+    if (o.status == SCATTER) return OUT_SCATTER;
+    if (o.status == SCATTER_EFFECTIVE) return OUT_REEMIT;
     return OUT_CONTINUE;
 }
 

@@ -128,6 +128,7 @@ int transport_blocks_per_sm(int minBlocks, bool fp32);
 void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in, uint32_t n,
                              uint32_t *nextIdx, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                              DevStats *st);
+void launch_fold_attenuation(cudaStream_t s, const Ctx &C, DevStats *st);   // after the transport, where C.att is set
 int refill_blocks_per_sm(int minBlocks, bool fp32);
 void launch_bank_to_local(cudaStream_t s, const Ctx &C, const Bank &src, const Bank &dst, uint32_t n,
                           uint32_t lo = 0);   // particles [lo, n)

@@ -1346,12 +1346,14 @@ __device__ __forceinline__ void block_stats_flush(const BlockStats &bs, DevStats
 // Form64T<4> is Form64T<1> without the DDMC branch.  Problems without
 // withDDMC run the variants without it: less code for the instruction cache,
 // whose misses bound the multigroup and polyhedral kernels.  TL is the
-// tally: SegmentTallyEg adds the group time averages (withEgTimeAvg),
+// tally: SegmentTallyRun serves the gray forms, SegmentTallyEg adds the group time averages (withEgTimeAvg),
 // SegmentTallyFixed sums in fixed point (reproducible tallies).
 template <int V, class TL = SegmentTally>
 struct Form64T {
+    static constexpr bool kTogether = true;
     using T = Track;
-    using Rng = PhiloxRng;
+    using Rng = PhiloxRng;       // bank visits
+    using Ring = PhiloxRing2;    // the persistent transport
     using Tally = TL;
     static __device__ __forceinline__ void load(const Ctx &C, const Bank &b, uint32_t q, T &t) {
         load_part(b, q, t.p);
@@ -1364,22 +1366,28 @@ struct Form64T {
                                                  uint32_t draw) {
         census_store64(b, q, t.p, pid, draw);
     }
-    template <class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        PhysOut o = physics_step<V>(C, t, rng, tal);
+        PhysOut o = physics_step<V, LATER>(C, t, rng, tal);
         if (o.errCode) { err = o.errCode; return OUT_ERROR; }
         usedRW = o.usedRW == 1;   // Random Walk jumps (2 marks a DDMC step)
+        if (o.status == CELL_MOVE && o.next != OUTSIDE) tal.leave(C, t.p.cell);
         int m = manager_handle<V == 2 || V == 5>(C, t, o);
         if (m == OUT_ERROR) err = STORM_DERR_NOT_ON_BOUNDARY;
         return m;
     }
+    // what a segment left (OUT_SCATTER, OUT_REEMIT)
+    template <class RNG>
+    static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int left) {
+        return finish64<V == 1 || V == 4>(C, t, rng, left == OUT_REEMIT);
+    }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.p.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.p.w; }
 };
-using Form64 = Form64T<0>;
+using Form64 = Form64T<0, SegmentTallyRun>;
 using Form64Full = Form64T<1>;
-using Form64Poly = Form64T<2>;
-using Form64PolyDDMC = Form64T<5>;   // Form64Poly with the DDMC branch
+using Form64Poly = Form64T<2, SegmentTallyRun>;
+using Form64PolyDDMC = Form64T<5, SegmentTallyRun>;   // Form64Poly with the DDMC branch
 using Form64Hydro = Form64T<3>;   // Form64Full with moving material
 using Form64MG = Form64T<4>;      // Form64Full without the DDMC branch
 using Form64FullEg = Form64T<1, SegmentTallyEg>;   // the multigroup forms with the group time averages
@@ -1392,13 +1400,14 @@ using Form64PolyFix = Form64T<2, SegmentTallyFixed>;
 using Form64PolyDDMCFix = Form64T<5, SegmentTallyFixed>;
 template <bool POLY, bool DDMC = true, class TL = SegmentTally>
 struct Form32T {
+    static constexpr bool kTogether = POLY;
     using T = Track32;
-    using Rng = PhiloxRng4;
+    using Rng = PhiloxRng4;      // bank visits
+    using Ring = PhiloxRing4;    // the persistent transport
     using Tally = TL;
     static __device__ __forceinline__ void load(const Ctx &C, const Bank &b, uint32_t q, T &t) {
         load32(b, q, t);
-        cell_ijk(C, t.cell, t.i, t.j, t.k);
-        t.cc = OUTSIDE;
+        begin_cell32<false, POLY>(C, t);
     }
     static __device__ __forceinline__ void keep(const Bank &b, uint32_t q, const T &t, uint32_t pid, uint32_t draw) {
         store32(b, q, t, pid, draw);
@@ -1407,19 +1416,23 @@ struct Form32T {
                                                  uint32_t draw) {
         census_store32(b, q, t, pid, draw);
     }
-    template <class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<false, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<false, LATER, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
         return m;
+    }
+    template <class RNG>
+    static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int) {
+        return finish32<false>(C, t, rng, true);
     }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.w; }
 };
-using Form32 = Form32T<false>;
-using Form32Lean = Form32T<false, false>;   // without the DDMC branch
-using Form32Poly = Form32T<true, false>;   // without the DDMC branch
-using Form32PolyDDMC = Form32T<true, true>;
+using Form32 = Form32T<false, true, SegmentTallyRun>;
+using Form32Lean = Form32T<false, false, SegmentTallyRun>;   // without the DDMC branch
+using Form32Poly = Form32T<true, false, SegmentTallyRun>;   // without the DDMC branch
+using Form32PolyDDMC = Form32T<true, true, SegmentTallyRun>;
 using Form32Fix = Form32T<false, true, SegmentTallyFixed>;   // reproducible tallies
 using Form32LeanFix = Form32T<false, false, SegmentTallyFixed>;
 using Form32PolyFix = Form32T<true, false, SegmentTallyFixed>;
@@ -1427,14 +1440,15 @@ using Form32PolyDDMCFix = Form32T<true, true, SegmentTallyFixed>;
 // The FP32-tracking form of a multigroup problem: the frequency rides along.
 template <bool DDMC = true, class TL = SegmentTally>
 struct Form32MGT {
+    static constexpr bool kTogether = true;
     using T = Track32;
-    using Rng = PhiloxRng4;
+    using Rng = PhiloxRng4;      // bank visits
+    using Ring = PhiloxRing4;    // the persistent transport
     using Tally = TL;
     static __device__ __forceinline__ void load(const Ctx &C, const Bank &b, uint32_t q, T &t) {
         load32(b, q, t);
         t.nu = load_nu32(b, q);
-        cell_ijk(C, t.cell, t.i, t.j, t.k);
-        t.cc = OUTSIDE;
+        begin_cell32<true, false>(C, t);
     }
     static __device__ __forceinline__ void keep(const Bank &b, uint32_t q, const T &t, uint32_t pid, uint32_t draw) {
         store32(b, q, t, pid, draw);
@@ -1444,11 +1458,16 @@ struct Form32MGT {
                                                  uint32_t draw) {
         census_store32_mg(b, q, t, pid, draw);
     }
-    template <class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<true, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<true, LATER, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
+        if (m == OUT_CONTINUE && t.nu < 0.0f) m = OUT_REEMIT;   // a Random Walk's upscatter
         return m;
+    }
+    template <class RNG>
+    static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int left) {
+        return finish32<true>(C, t, rng, left == OUT_SCATTER);
     }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.w; }
@@ -1487,7 +1506,7 @@ __device__ __forceinline__ void visit_bank(const Ctx &C, const Bank &in, uint32_
                 tal.enter(cell0);
                 ++s;
                 int usedRW = 0, err = 0;
-                outcome = F::seg(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
                 rw += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
@@ -1540,43 +1559,65 @@ __global__ void __launch_bounds__(256, MINB) k_transport32(Ctx C, Bank in, const
 // The whole HandleAll loop in one launch.  Every lane holds one history; a lane
 // whose particle reaches census, escapes or is cut off writes it out and takes
 // the next unstarted particle, so lanes do not idle behind the longest history
-// of their warp.  Each warp takes unstarted particles from the bank in chunks of
-// REFILL_CHUNK (one global atomic per chunk) and hands them to its empty lanes
-// between bursts of `burst` segments.  Per-lane totals (segments, deposits,
-// census energy) live in the lane's own shared-memory slot until the end.  A
-// history longer than maxSegs raises STORM_DERR_HISTORY_CAP and stops.
-constexpr uint32_t REFILL_CHUNK = 32;
+// of their warp.  Each warp takes unstarted particles from the bank in chunks
+// (one global atomic per chunk) and hands them to its empty lanes between bursts
+// of `burst` segments.  The bank is in cell order, so a chunk of 64 keeps a
+// warp's cells together longer than one of 32 (64^3 gray cube: 5.85 to 5.69 ms
+// FP32, 20.2 to 19.6 ms FP64); longer ones leave a warp with a cell's long
+// histories at the end (256: 40^3 multigroup 1.0 to 1.5 ms), and the share shrinks
+// with what is left.  Per-lane totals live in the lane's own shared-memory slot
+// until the end, counts of ended histories in warp-uniform registers.  A history
+// longer than maxSegs raises STORM_DERR_HISTORY_CAP and stops.
+// What bounds it: instruction issue (77 % of the slots, 20 of 32 lanes, gray FP32)
+// or instruction fetch and divergence (FP64, multigroup), dependent loads of the
+// face planes on polyhedral meshes; a problem of few cells or few, long
+// histories by the chain of its longest history.
+// Transport of the second step, before and after the rings, the run tally, the
+// finish and the leaner refill: 64^3 gray cube, 4.2e8 segments, FP32 7.5 to 5.8 ms,
+// FP64 19.6 to 18.3; 24^3, 2.1e7 segments, FP32 0.78 to 0.50; 100-cell slab, 8e6
+// segments, FP64 3.1 to 1.4; 72^3 x 64 groups, 2.6e7 segments, FP32 2.77 to 1.90;
+// Voronoi 4e4 cells, 8.6e7 segments, FP32 6.4 to 6.2.
+constexpr uint32_t REFILL_CHUNK_MAX = 64;
 
 template <class F, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, uint32_t n, uint32_t *nextIdx, CensusBank cen,
                                                                  uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                                                                  DevStats *st) {
     __shared__ BlockStats bs;
-    __shared__ double sDep[256], sCen[256];
+    __shared__ double sDep[256], sCen[256], sEsc[256];
     __shared__ uint32_t sSegs[256], sRw[256];
+    using Ring = typename F::Ring;
+    __shared__ uint32_t ring[Ring::kWords * 256];
     const unsigned tid = threadIdx.x;
-    sDep[tid] = 0.0; sCen[tid] = 0.0; sSegs[tid] = 0; sRw[tid] = 0;
+    sDep[tid] = 0.0; sCen[tid] = 0.0; sEsc[tid] = 0.0; sSegs[tid] = 0; sRw[tid] = 0;
     block_stats_zero(bs);
     const unsigned lane = tid & 31;
     const unsigned lt = lanemask_lt();
+    using Tally = typename F::Tally;
     typename F::T t;
-    typename F::Rng rng;
+    Ring rng;
+    Tally tal;
+    if constexpr (Tally::kRun) tal.begin(&sDep[tid]);   // holds a history's tallies back while it stays in its cell
     uint32_t pid = 0, segsThis = 0;
     bool has = false;
     uint32_t cBase = 0, cLeft = 0;   // warp-uniform: this warp's chunk of unstarted particles
     bool drained = false;            // warp-uniform: the bank counter has passed n
+    uint32_t nEsc = 0, nCut = 0, nDone = 0;   // warp-uniform: histories ended so far, by outcome
     for (;;) {
         unsigned need = __ballot_sync(FULL, !has);
         while (need) {
             if (cLeft == 0) {
                 if (drained) break;
+                // a share of what was left at this warp's last chunk
+                const uint32_t share = (n - cBase) / (gridDim.x * 16u);
+                const uint32_t chunk = min(max(share & ~31u, 32u), REFILL_CHUNK_MAX);
                 uint32_t b = 0;
-                if (lane == 0) b = atomicAdd(nextIdx, REFILL_CHUNK);
+                if (lane == 0) b = atomicAdd(nextIdx, chunk);
                 b = __shfl_sync(FULL, b, 0);
                 if (b >= n) { drained = true; break; }
-                if (n - b <= REFILL_CHUNK) drained = true;
+                if (n - b <= chunk) drained = true;
                 cBase = b;
-                cLeft = min(REFILL_CHUNK, n - b);
+                cLeft = min(chunk, n - b);
             }
             const uint32_t take = min(static_cast<uint32_t>(__popc(need)), cLeft);
             const uint32_t rank = __popc(need & lt);
@@ -1584,7 +1625,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                 const uint32_t q = cBase + rank;
                 F::load(C, in, q, t);
                 pid = in.pid[q];
-                rng.init(C.seedLo, C.seedHi, TAG_TRANSPORT, C.step, pid, in.draw[q]);
+                rng.init(C, ring, pid, in.draw[q]);
                 segsThis = 0;
                 has = true;
             }
@@ -1594,58 +1635,127 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
         }
         if (!__any_sync(FULL, has)) break;
         int outcome = OUT_CONTINUE;
-        if (has) {
-            typename F::Tally tal;
-            tal.init(C.eint, C.eradAvg, C.perCellCounters ? C.segs : nullptr);
-            if constexpr (std::is_same_v<typename F::Tally, SegmentTallyFixed>) tal.init_fixed(C);
-            uint32_t segs = 0, rws = 0;
+        if constexpr (!Tally::kRun) tal.init(C.eint, C.eradAvg, C.perCellCounters ? C.segs : nullptr);
+        if constexpr (std::is_same_v<Tally, SegmentTallyFixed>) tal.init_fixed(C);
+        const uint32_t before = segsThis;
+        uint32_t rws = 0;
+        // FP64, multigroup and polyhedral segments are long, and lanes that part at
+        // an event drift through the code on their own: there the lanes of a warp
+        // start each segment together and finish their scatters together (64^3
+        // gray FP64 19.6 to 18.3 ms, 72^3 multigroup FP32 1.99 to 1.90, Voronoi FP64
+        // 3.02 to 2.85).  The gray Cartesian FP32 segment is too short to gain by it
+        // (5.7 to 6.2).  Holding scatters back until several lanes have one loses:
+        // the waiting lanes idle (18.7 ms with every scatter at once, 19.3 and 20.7
+        // with four and eight).
+        if constexpr (F::kTogether) {
+            bool live = has;
+            for (uint32_t b = 0; b < burst; ++b) {
+                int left = OUT_CONTINUE;
+                if (live) {
+                    const uint32_t cell0 = F::cell(t);
+                    tal.enter(cell0);
+                    ++segsThis;
+                    int usedRW = 0, err = 0;
+                    outcome = F::template seg<true>(C, t, rng, tal, usedRW, err);
+                    rws += usedRW;
+                    if (outcome >= OUT_SCATTER) {
+                        left = outcome;
+                        outcome = OUT_CONTINUE;
+                    }
+                    if (outcome == OUT_ERROR) {
+                        raise_error(C, err, cell0, pid);
+                    } else if (outcome == OUT_CONTINUE && segsThis >= maxSegs) {
+                        raise_error(C, STORM_DERR_HISTORY_CAP, cell0, pid);
+                        outcome = OUT_ERROR;
+                    }
+                    live = outcome == OUT_CONTINUE;
+                }
+                __syncwarp();
+                if (live && left != OUT_CONTINUE && !F::finish(C, t, rng, left)) {
+                    raise_error(C, STORM_DERR_MG_SAMPLE, F::cell(t), pid);
+                    outcome = OUT_ERROR;
+                    live = false;
+                }
+                __syncwarp();
+            }
+        } else if (has) {
             for (uint32_t b = 0; b < burst; ++b) {
                 const uint32_t cell0 = F::cell(t);
                 tal.enter(cell0);
-                ++segs;
+                ++segsThis;
                 int usedRW = 0, err = 0;
-                outcome = F::seg(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
                 rws += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
                     break;
                 }
-                if (++segsThis >= maxSegs) {
+                if (segsThis >= maxSegs) {
                     raise_error(C, STORM_DERR_HISTORY_CAP, cell0, pid);
                     outcome = OUT_ERROR;
                     break;
                 }
             }
-            sSegs[tid] += segs;
+        }
+        if (has) {
+            sSegs[tid] += segsThis - before;
             if (rws) sRw[tid] += rws;
-            sDep[tid] += tal.depSum;
-            if (outcome == OUT_ESCAPE) { atomicAdd(&bs.escaped, 1ull); atomicAdd(&bs.eEscaped, F::weight(t)); }
-            else if (outcome == OUT_CUTOFF) atomicAdd(&bs.cutoff, 1ull);
+            if constexpr (!Tally::kRun) sDep[tid] += tal.depSum;
+            if (outcome == OUT_ESCAPE) sEsc[tid] += F::weight(t);
             else if (outcome == OUT_CENSUS) sCen[tid] += F::weight(t);
         }
-        const bool cens = has && outcome == OUT_CENSUS;
-        const unsigned mC = __ballot_sync(FULL, cens);
-        if (mC) {
-            uint32_t bC = 0;
-            if (lane == 0) {
-                bC = atomicAdd(nCen, __popc(mC));
-                atomicAdd(&bs.census, static_cast<unsigned long long>(__popc(mC)));
+        const unsigned ended = __ballot_sync(FULL, has && outcome != OUT_CONTINUE);
+        if (ended) {
+            const bool cens = has && outcome == OUT_CENSUS;
+            const unsigned mC = __ballot_sync(FULL, cens);
+            nEsc += __popc(__ballot_sync(FULL, has && outcome == OUT_ESCAPE));
+            nCut += __popc(__ballot_sync(FULL, has && outcome == OUT_CUTOFF));
+            if (mC) {
+                nDone += __popc(mC);
+                uint32_t bC = 0;
+                if (lane == 0) bC = atomicAdd(nCen, __popc(mC));
+                bC = __shfl_sync(FULL, bC, 0);
+                if (cens) F::store(cen, bC + __popc(mC & lt), t, pid, rng.draw);
             }
-            bC = __shfl_sync(FULL, bC, 0);
-            if (cens) F::store(cen, bC + __popc(mC & lt), t, pid, rng.draw);
+            if (has && outcome != OUT_CONTINUE) {
+                tal.leave(C, F::cell(t));
+                has = false;
+            }
         }
-        if (has && outcome != OUT_CONTINUE) has = false;
     }
     // per-lane totals -> block
     const uint32_t segs = warp_sum(sSegs[tid]), rws = warp_sum(sRw[tid]);
-    const double dep = warp_sum(sDep[tid]), eC = warp_sum(sCen[tid]);
+    const double dep = warp_sum(sDep[tid]), eC = warp_sum(sCen[tid]), eE = warp_sum(sEsc[tid]);
     if (lane == 0) {
+        if (nEsc) atomicAdd(&bs.escaped, static_cast<unsigned long long>(nEsc));
+        if (nCut) atomicAdd(&bs.cutoff, static_cast<unsigned long long>(nCut));
+        if (nDone) atomicAdd(&bs.census, static_cast<unsigned long long>(nDone));
+        if (eE != 0.0) atomicAdd(&bs.eEscaped, eE);
         if (segs) atomicAdd(&bs.segments, static_cast<unsigned long long>(segs));
         if (rws) atomicAdd(&bs.rwSteps, static_cast<unsigned long long>(rws));
         if (dep != 0.0) atomicAdd(&bs.eDeposited, dep);
         if (eC != 0.0) atomicAdd(&bs.eCensusPre, eC);
     }
     block_stats_flush(bs, st);
+}
+
+// The gray transports' attenuation (SegmentTallyRun) to the material and, times
+// -1 / the cell's absorption rate, to the radiation tally; cleared for the next step.
+__global__ void k_fold_attenuation(Ctx C, DevStats *st) {
+    double dep = 0.0;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < C.ncells; c += gridDim.x * blockDim.x) {
+        const double v = C.att[c];
+        if (v == 0.0) continue;
+        const double invRate = C.fp32 ? static_cast<double>(C.phys32[c].w) : C.phys[c].z;
+        if (!C.noFeedback) {
+            C.eint[c] += v;
+            dep += v;
+        }
+        C.eradAvg[c] -= v * invRate;
+        C.att[c] = 0.0;
+    }
+    dep = warp_sum(dep);
+    if ((threadIdx.x & 31) == 0 && dep != 0.0) atomicAdd(&st->eDeposited, dep);
 }
 
 // ------------------------------------------------------------------ comb
@@ -3618,6 +3728,9 @@ void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const
     else if (C.groups >= 2 && !C.withDDMC) refill_launch<Form64MG>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
     else if (C.groups >= 2 || C.withDDMC) refill_launch<Form64Full>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
     else refill_launch<Form64>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
+}
+void launch_fold_attenuation(cudaStream_t s, const Ctx &C, DevStats *st) {
+    k_fold_attenuation<<<grid_for(C.ncells, 256, 8192), 256, 0, s>>>(C, st);
 }
 template <class F>
 static int refill_occ(int minBlocks) {

@@ -128,6 +128,7 @@ struct StormHandle {
     std::vector<uint64_t> shardCensus;   // census particles per shard after the last comb (every shard)
     uint64_t nCenGlobal = 0, nCellEmitGlobal = 0, nFaceEmitGlobal = 0;   // this step's global counts
     double *dep = nullptr;           // this handle's material deposits of the step (N)
+    double *att = nullptr;           // gray problems: the transport's attenuation per cell (SegmentTallyRun)
     double4 *vel = nullptr;          // moving material: (vx, vy, vz, gamma) per cell
     double *egAvg = nullptr;         // group time averages (with_eg_time_avg): ncells x groups
     unsigned long long *fixMat = nullptr, *fixRad = nullptr;   // reproducible tallies: 4 limbs per cell
@@ -1102,6 +1103,10 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     H2D(A.mass, d->mass, N);
     H2D(A.eint, d->internal_energy, N);
     H2D(A.ceint, d->cell_internal_energy ? d->cell_internal_energy : d->internal_energy, N);
+    if (d->groups < 2 && !d->with_hydro) {
+        ALLOC(h->att, N);
+        ZERO(h->att, N * sizeof(double));
+    }
     ZERO(A.eradAvg, N * sizeof(double));
     ZERO(A.eradCensus, N * sizeof(double));
     ZERO(A.sigS, N * sizeof(double));
@@ -1306,6 +1311,12 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     C.rwDiffPerReach = C.rwMinParticle > 0.0 ? static_cast<float>(C.clight / (3.0 * C.rwMinParticle)) : 0.0f;
     C.seedLo = static_cast<uint32_t>(d->seed);
     C.seedHi = static_cast<uint32_t>(d->seed >> 32);
+    C.nxMagic = static_cast<uint32_t>((1ull << 32) / C.nx + 1);
+    C.nyMagic = static_cast<uint32_t>((1ull << 32) / C.ny + 1);
+    for (uint32_t r = 0; r < 10; ++r) {
+        C.philoxKey[2 * r] = C.seedLo + r * 0x9E3779B9u;
+        C.philoxKey[2 * r + 1] = C.seedHi + r * 0xBB67AE85u;
+    }
     C.step = 0;
     C.phys = A.phys;
     C.phys32 = A.phys32;
@@ -1313,7 +1324,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     C.hx = h->hx; C.hy = h->hy; C.hz = h->hz;
     C.invC = 1.0 / d->clight;
     C.sigA = A.sigA; C.sigS = A.sigS; C.fleck = A.fleck; C.rwSigT = A.rwSigT; C.rwElig = A.rwElig;
-    C.eint = A.eint; C.eradAvg = A.eradAvg; C.segs = h->segs;
+    C.eint = A.eint; C.eradAvg = A.eradAvg; C.att = h->att; C.segs = h->segs;
     C.err = h->dErr;
 
     if (build_face_sources(h) != STORM_OK) return fail(STORM_ERR_CUDA);
@@ -1350,7 +1361,7 @@ int storm_cuda_destroy(StormHandle *h) {
                   h->ddmcRate, h->ddmcCut, h->ddmc32, h->stratBounds, h->stratBinW, h->stratStart,
                   h->runCursor, h->runScan, h->longRuns, h->bucketFlags,
                   h->cfo, h->cfN, h->cfP, h->cfNext, h->cfFace, h->mpx, h->mpy, h->mpz, h->fvo, h->fvi, h->vtx,
-                  h->chord, h->cfN32, h->dep, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds,
+                  h->chord, h->cfN32, h->dep, h->att, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds,
                   h->vel, h->mom, h->ddmcCum32, h->cfA, h->egAvg, h->fixMat, h->fixRad, h->tetOff, h->tetCum,
                   h->tetAT};
     for (void *p : ps) device_pool().free(p);
@@ -1616,6 +1627,10 @@ int storm_cuda_phase_transport(StormHandle *h) {
                                     h->burst, maxSegs, h->dStats);
             if (h->profiling) CK(cudaEventRecord(h->evPool[1], h->stream));
             ++h->launches;
+            if (h->att) {
+                launch_fold_attenuation(h->stream, h->C, h->dStats);
+                ++h->launches;
+            }
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(h->evTransport1, h->stream));
@@ -2286,6 +2301,10 @@ static int step_host_overlapped(StormHandle *h, double dt, const StormParticlesS
                                 static_cast<uint32_t>(hi), h->counts + 1, h->bankC, nCen, h->burst, maxSegs,
                                 h->dStats);
         h->launches += 2;
+    }
+    if (h->att) {
+        launch_fold_attenuation(h->stream, h->C, h->dStats);
+        ++h->launches;
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->evTransport1, h->stream));
