@@ -2515,14 +2515,17 @@ int storm_cuda_get_cell_arrays(StormHandle *h, double *T, double *eint, double *
     double *dst[] = {T, eint, eradAvg, eradCensus, sigA, fleck};
     for (int q = 0; q < 6; ++q)
         if (dst[q]) CK(cudaMemcpyAsync(dst[q], src[q], N * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    std::vector<uint32_t> s32;
-    if (segs) {
-        s32.resize(N);
-        CK(cudaMemcpyAsync(s32.data(), h->segs, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    }
+    // the 32-bit counters go to the upper half of the caller's array and are widened
+    // from there, front to back: element q is read at or behind where it is written
+    unsigned char *upper = segs ? reinterpret_cast<unsigned char *>(segs) + N * sizeof(uint32_t) : nullptr;
+    if (segs) CK(cudaMemcpyAsync(upper, h->segs, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     if (segs)
-        for (size_t q = 0; q < N; ++q) segs[q] = s32[q];
+        for (size_t q = 0; q < N; ++q) {
+            uint32_t v;
+            std::memcpy(&v, upper + q * sizeof(uint32_t), sizeof(v));
+            segs[q] = v;
+        }
     return STORM_OK;
 }
 
