@@ -107,6 +107,7 @@ void launch_allocate_if(cudaStream_t s, const Ctx &C, const CellArrays &A, const
                         const int32_t *onlyIf);
 void launch_emission_debit(cudaStream_t s, const Ctx &C, const CellArrays &A, DevStats *st);
 void launch_scan_u64(cudaStream_t s, const uint64_t *in, uint32_t n, uint64_t *out, uint64_t *tileSums, uint64_t *total);
+uint32_t scan_launches(uint32_t n);   // kernels of a scan of n words
 void launch_emit_cells(cudaStream_t s, const Ctx &C, const CellArrays &A, const uint64_t *offsets, uint64_t eBegin,
                        uint64_t count, const Bank &b, uint32_t bankBase, uint32_t pidBase, double dt, DevStats *st);
 void launch_ddmc_rates(cudaStream_t s, const Ctx &C, const CellArrays &A);
@@ -116,7 +117,8 @@ void launch_strat_sums(cudaStream_t s, const double *wS, const uint32_t *start, 
                        double *binW, double *cellW);
 void launch_strat_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const StratParams &S, const double *wS,
                        const uint32_t *start, const double *binW, const double *cellW, const double *Wtot,
-                       uint32_t *pCount, double *pWeight, uint64_t *cellCount, double *eradCensus, DevStats *st);
+                       uint32_t *pCount, double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
+                       DevStats *st);
 void launch_face_spectra(cudaStream_t s, const Ctx &C, double *cdf);
 void launch_set_u32(cudaStream_t s, uint32_t *p, uint32_t v);
 void launch_poly_tets(cudaStream_t s, const Ctx &C, const uint32_t *tetOff, double *tetCum, uint2 *tetAT);
@@ -143,7 +145,6 @@ void launch_bucket_sort(cudaStream_t s, const Ctx &C, const CensusBank &cen, con
                         int pidBits, uint32_t nRuns, uint32_t *start, uint32_t *cursor, uint64_t *scanSums,
                         uint64_t *outKeys, uint32_t *outVals, double *wS, uint32_t *longRuns, uint32_t longCap,
                         uint32_t *flags, const double *wc = nullptr);
-void launch_mask_count_upto(cudaStream_t s, const uint32_t *pCount, uint32_t n, const uint32_t *nValid, uint64_t *out);
 size_t bucket_scan_words(uint32_t len);
 uint32_t bucket_long_capacity(uint32_t n);
 void launch_sorted_weights(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, uint32_t n,
@@ -154,14 +155,14 @@ void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *sta
 void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out);
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
-                      uint64_t *cellCount, double *eradCensus, DevStats *st);
+                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st);
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,
-                      const uint64_t *pOffset, const Bank &out);
+                      const uint32_t *pOff, const uint64_t *groupOff, const Bank &out);
 void launch_comb_emit_out(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx,
                           const uint64_t *sortedKeys, int pidBits, uint32_t bins, uint32_t nValid, uint32_t total,
-                          const uint32_t *pCount, const double *pWeight, const uint64_t *pOffset, uint32_t *src,
-                          uint32_t *tileMax, const Bank &out);
+                          const uint32_t *pCount, const double *pWeight, const uint32_t *pOff, const uint64_t *groupOff,
+                          uint32_t *src, const Bank &out);
 void launch_allocate_checked(cudaStream_t s, const Ctx &C, const CellArrays &A, const double *total,
                              uint64_t newPerCell, double rel, int32_t *ambiguous);
 size_t radix_scratch_words(uint32_t n);
@@ -177,11 +178,10 @@ void launch_shard_pack_runs(cudaStream_t s, const double *runW, const uint32_t *
 void launch_shard_cell_weights(cudaStream_t s, const double *x, uint32_t ncells, uint32_t shards, double *Wc);
 void launch_comb_plan_sharded(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS,
                               const uint32_t *start, const double *x, const double *Wc, const double *Wtot,
-                              uint32_t lo, uint32_t hi, uint32_t *pCount, double *pWeight, double *eradCensus,
-                              DevStats *st);
-void launch_shard_pack_census(cudaStream_t s, const uint64_t *pOff, const uint64_t *total, const uint32_t *start,
-                              uint32_t n, uint32_t ncells, uint32_t shards, uint32_t lo, uint32_t hi,
-                              const double *eradCensus, double *x);
+                              uint32_t lo, uint32_t hi, uint32_t *pCount, double *pWeight, uint32_t *pOff,
+                              uint64_t *runCount, double *eradCensus, DevStats *st);
+void launch_shard_pack_census(cudaStream_t s, const uint64_t *runOff, uint32_t ncells, uint32_t shards, uint32_t lo,
+                              uint32_t hi, const double *eradCensus, double *x);
 void launch_add_into(cudaStream_t s, double *y, const double *x, uint32_t n);
 void launch_to_float(cudaStream_t s, const double *src, float *dst, uint32_t n);
 void launch_poststep(cudaStream_t s, const Ctx &C, const CellArrays &A, const OpacityEos &M, double dt);

@@ -25,6 +25,21 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// Adds v over the block's threads (256 at most) to *to with one atomic: a warp's
+// atomic each made 8192 of them wait on one address at 64^3 cells (16 us of a 16 us
+// kernel).  Every thread of the block calls it.
+__device__ __forceinline__ void block_add(double v, double *to) {
+    __shared__ double part[8];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (unsigned w = 0; w < blockDim.x / 32; ++w) s += part[w];
+        if (s != 0.0) atomicAdd(to, s);
+    }
+}
+
 // ------------------------------------------------------------------ bank access
 __device__ __forceinline__ void load_part(const Bank &b, uint32_t q, PartReg &p) {
     p.x = b.x[q]; p.y = b.y[q]; p.z = b.z[q];
@@ -729,8 +744,7 @@ __global__ void k_emission_debit(Ctx C, CellArrays A, DevStats *st) {
         }
         deb += E;
     }
-    deb = warp_sum(deb);
-    if ((threadIdx.x & 31) == 0 && deb != 0.0) atomicAdd(&st->eDebit, deb);
+    block_add(deb, &st->eDebit);
 }
 
 // ------------------------------------------------------------------ exclusive scan (uint64)
@@ -782,6 +796,28 @@ __global__ void k_scan_sums(uint64_t *tileSums, uint32_t ntiles, uint64_t *total
         __syncthreads();
     }
     if (threadIdx.x == 0) *total = carry;
+}
+// A short scan by one block in one launch: a pass of 1024 costs about half a
+// launch, so up to eight of them are cheaper than the other two launches.
+constexpr uint32_t SCAN_ONE_BLOCK = 8192;
+__global__ void __launch_bounds__(1024) k_scan_block(const uint64_t *in, uint32_t n, uint64_t *out, uint64_t *total) {
+    __shared__ uint64_t sh[32];
+    __shared__ uint64_t last;
+    uint64_t carry = 0;
+    for (uint32_t base = 0; base < n; base += 1024) {
+        const uint32_t q = base + threadIdx.x;
+        const uint64_t v = q < n ? in[q] : 0;
+        const uint64_t inc = block_scan_incl(v, sh);
+        if (q < n) out[q] = carry + inc - v;
+        if (threadIdx.x == 1023) last = inc;
+        __syncthreads();
+        carry += last;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[n] = carry;
+        *total = carry;
+    }
 }
 __global__ void k_scan_add(uint64_t *out, uint32_t n, const uint64_t *tileSums, const uint64_t *total) {
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1754,8 +1790,7 @@ __global__ void k_fold_attenuation(Ctx C, DevStats *st) {
         C.eradAvg[c] -= v * invRate;
         C.att[c] = 0.0;
     }
-    dep = warp_sum(dep);
-    if ((threadIdx.x & 31) == 0 && dep != 0.0) atomicAdd(&st->eDeposited, dep);
+    block_add(dep, &st->eDeposited);
 }
 
 // ------------------------------------------------------------------ comb
@@ -1803,7 +1838,8 @@ __device__ __forceinline__ uint32_t shard_of_pid(const Ctx &C, uint32_t pid) {
 
 // The cell of a comb run: runs are (shard, cell) when sharded, else (cell, bin).
 __device__ __forceinline__ uint32_t cell_of_run(const Ctx &C, uint64_t run, uint32_t bins) {
-    return C.shards > 1 ? static_cast<uint32_t>(run % C.ncells) : static_cast<uint32_t>(run / bins);
+    return C.shards > 1 ? static_cast<uint32_t>(run % C.ncells)
+                        : (bins == 1 ? static_cast<uint32_t>(run) : static_cast<uint32_t>(run / bins));
 }
 
 __global__ void k_comb_keys(Ctx C, CensusBank cen, uint32_t n, uint64_t *keys, uint32_t *vals, uint32_t combKey,
@@ -1858,6 +1894,22 @@ __global__ void k_scan32_tiles(uint32_t *v, uint32_t n, uint64_t *tileSums) {
     uint64_t inc = block_scan_incl(x, sh);
     if (q < n) v[q] = static_cast<uint32_t>(inc - x);
     if (threadIdx.x == blockDim.x - 1) tileSums[blockIdx.x] = inc;
+}
+// the same of 32-bit words in place, by one block
+__global__ void __launch_bounds__(1024) k_scan32_block(uint32_t *v, uint32_t n) {
+    __shared__ uint64_t sh[32];
+    __shared__ uint64_t last;
+    uint64_t carry = 0;
+    for (uint32_t base = 0; base < n; base += 1024) {
+        const uint32_t q = base + threadIdx.x;
+        const uint64_t x = q < n ? v[q] : 0;
+        const uint64_t inc = block_scan_incl(x, sh);
+        if (q < n) v[q] = static_cast<uint32_t>(carry + inc - x);
+        if (threadIdx.x == 1023) last = inc;
+        __syncthreads();
+        carry += last;
+        __syncthreads();
+    }
 }
 __global__ void k_scan32_add(uint32_t *v, uint32_t n, const uint64_t *tileSums) {
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1969,9 +2021,11 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint64_t *kin, 
 // is the radix sort's.  A run longer than BUCKET_BLOCK_MAX keys raises a flag,
 // and the caller falls back to the radix sort.
 
-constexpr uint32_t BUCKET_WARP_MAX = 512;     // runs up to this length: one warp (registers, then 4 KB of shared memory)
-constexpr uint32_t BUCKET_BLOCK_MAX = 8192;   // longer runs up to this length: one block of 256, 64 KB
+constexpr uint32_t BUCKET_WARP_MAX = 512;     // runs up to this length: one warp (registers to 128, then 4 KB of shared memory)
+constexpr uint32_t BUCKET_WARP_FEW = 128;     // the same where there are too few runs to fill the chip with warps
+constexpr uint32_t BUCKET_BLOCK_MAX = 8192;   // longer runs up to this length: one block, 64 KB
 constexpr int BUCKET_WARPS = 8;
+constexpr uint32_t BUCKET_LONG_THREADS = 1024;
 
 // keys of run nRuns (zero weight, outside the mesh) and any run index beyond it share the last bucket
 __device__ __forceinline__ uint32_t bucket_run(uint64_t key, int pidBits, uint32_t nRuns) {
@@ -2214,7 +2268,8 @@ __global__ void __launch_bounds__(32 * BUCKET_WARPS) k_bucket_sort_runs(Ctx C, C
                                                                         uint64_t *keys, uint32_t *vals, double *wS,
                                                                         const uint32_t *start, uint32_t nRuns,
                                                                         int pidBits, uint32_t *longRuns,
-                                                                        uint32_t *nLong, uint32_t longCap) {
+                                                                        uint32_t *nLong, uint32_t longCap,
+                                                                        uint32_t warpMax) {
     __shared__ uint64_t sm[BUCKET_WARPS][BUCKET_WARP_MAX];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint64_t *sw = sm[wid];
@@ -2234,7 +2289,7 @@ __global__ void __launch_bounds__(32 * BUCKET_WARPS) k_bucket_sort_runs(Ctx C, C
         } else if (len <= 128) {
             if (pidBits <= 24) warp_sort_run32<4>(C, cen, keys, vals, wS, wc, b, len, r, pidBits, hashMask, lane);
             else warp_sort_run<4>(C, cen, keys, vals, wS, wc, b, len, r, pidBits, hashMask, lane);
-        } else if (len <= BUCKET_WARP_MAX) {
+        } else if (len <= warpMax) {
             uint32_t P = 256;
             while (P < len) P <<= 1;
             for (uint32_t i = lane; i < P; i += 32)
@@ -2257,8 +2312,10 @@ __global__ void __launch_bounds__(32 * BUCKET_WARPS) k_bucket_sort_runs(Ctx C, C
 }
 
 // The listed runs, one block each (dynamic shared memory: BUCKET_BLOCK_MAX words).
+// A stage of the network is a few compares a thread and a barrier, so the more
+// threads the better: 256 took 276 us on a slab whose longest cell holds thousands.
 // A run longer than BUCKET_BLOCK_MAX, or more listed runs than longCap, sets *tooLong.
-__global__ void __launch_bounds__(256) k_bucket_sort_long(Ctx C, CensusBank cen, const double *wc, uint64_t *keys,
+__global__ void __launch_bounds__(BUCKET_LONG_THREADS) k_bucket_sort_long(Ctx C, CensusBank cen, const double *wc, uint64_t *keys,
                                                           uint32_t *vals,
                                                           double *wS, const uint32_t *start, int pidBits,
                                                           const uint32_t *longRuns, const uint32_t *nLong,
@@ -2416,7 +2473,15 @@ __global__ void k_comb_cell_sums_thread(const double *wS, const uint32_t *start,
 __global__ void k_blocked_sum(const double *v, uint32_t n, double *out) {
     __shared__ double part[1024];
     double s = 0.0;
-    for (uint32_t q = threadIdx.x; q < n; q += 1024) s += v[q];
+    uint32_t q = threadIdx.x;
+    for (; q + 7 * 1024 < n; q += 8 * 1024) {   // eight loads on their way at a time, added in order
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = v[q + u * 1024];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += x[u];
+    }
+    for (; q < n; q += 1024) s += v[q];
     part[threadIdx.x] = s;
     __syncthreads();
     for (uint32_t w = 512; w >= 1; w >>= 1) {
@@ -2498,13 +2563,6 @@ __device__ __noinline__ double add_repeated(double s, double x, uint64_t n) {
     return s;
 }
 
-// the same for the few copies of a split particle
-__device__ __forceinline__ double add_copies(double s, double x, uint32_t n) {
-    if (n > 32) return add_repeated(s, x, n);
-    for (; n > 0; --n) s += x;
-    return s;
-}
-
 // Per cell (:161-226): the number of copies of each sorted particle, the weight
 // of those copies, and the cell's census radiation energy summed in output order
 // (RadiationIMC::postStep :2013-2016).  A warp takes its batch of cells one after
@@ -2513,14 +2571,16 @@ __device__ __forceinline__ double add_copies(double s, double x, uint32_t n) {
 // the census energy is that many times the same weight (add_repeated).  In a cell
 // that is kept or split the energy is the running weight, too, up to the first
 // particle that is split; only from there on is there a serial chain, over the
-// copies, walked from shared memory.
+// copies, which are laid out in shared memory for it.  pOff: a particle's first
+// copy among its cell's.
 __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams P, const double *wS,
                                                                const uint32_t *start, const double *W,
                                                                const double *upTo, const double *Wtot,
-                                                               uint32_t *pCount, double *pWeight, uint64_t *cellCount,
-                                                               double *eradCensus, DevStats *st, uint32_t batch) {
-    __shared__ __align__(16) double stage[WALK_WARPS][32];
-    __shared__ __align__(16) uint32_t copies[WALK_WARPS][32];
+                                                               uint32_t *pCount, double *pWeight, uint32_t *pOff,
+                                                               uint64_t *cellCount, double *eradCensus, DevStats *st,
+                                                               uint32_t batch) {
+    constexpr uint32_t COPIES = 256;   // copies of 32 particles that are laid out for the chain
+    __shared__ __align__(16) double stage[WALK_WARPS][COPIES + 8];
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -2528,7 +2588,6 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
     const bool none = tot == 0.0 || !isfinite(tot);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double *x = stage[wid];
-    uint32_t *nx = copies[wid];
     const uint32_t c = (blockIdx.x * WALK_WARPS + wid) * batch + lane;
     const bool mine = lane < batch && c < C.ncells;
     const uint32_t a = mine ? start[c] : 0u, b = mine ? start[c + 1] : 0u;
@@ -2565,40 +2624,47 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
                     ns = static_cast<uint64_t>(ceil(w / ideal));
                     ws = w / static_cast<double>(ns);
                 }
+                uint64_t upto = ns;   // copies of this chunk's particles up to this one
+                if (cut) {
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint64_t y = __shfl_up_sync(FULL, upto, o);
+                        if (static_cast<int>(lane) >= o) upto += y;
+                    }
+                } else {
+                    upto = min(lane + 1, rb - base);
+                }
+                const uint64_t chunk = __shfl_sync(FULL, upto, 31);
                 if (in) {
                     pCount[q] = split ? static_cast<uint32_t>(ns) : (1u | KEEP);
                     pWeight[q] = ws;
+                    pOff[q] = static_cast<uint32_t>(made + upto - ns);
                 }
-                made += cut ? warp_sum(ns) : min(32u, rb - base);
-                uint32_t i = 0;
+                int from = 0;
                 if (!chain && cut) {   // the energy up to the first split particle is the running weight
-                    i = __ffs(cut) - 1;
+                    from = __ffs(cut) - 1;
                     chain = true;
-                    e = base + i > ra ? upTo[base + i - 1] : 0.0;
+                    e = base + from > ra ? upTo[base + from - 1] : 0.0;
                 }
                 if (chain) {
-                    x[lane] = ws;
-                    nx[lane] = static_cast<uint32_t>(ns < 0xFFFFFFFFull ? ns : 0xFFFFFFFFull);
-                    __syncwarp();
-                    for (; (i & 3u) != 0; ++i) e = add_copies(e, x[i], nx[i]);
-                    for (; i < 32; i += 4) {   // nothing is added beyond the run: no copies there
-                        const double2 d0 = *reinterpret_cast<const double2 *>(x + i);
-                        const double2 d1 = *reinterpret_cast<const double2 *>(x + i + 2);
-                        const uint4 k = *reinterpret_cast<const uint4 *>(nx + i);
-                        if ((k.x | k.y | k.z | k.w) <= 1u) {
-                            e += d0.x;
-                            e += d0.y;
-                            e += d1.x;
-                            e += d1.y;
-                        } else {
-                            e = add_copies(e, d0.x, k.x);
-                            e = add_copies(e, d0.y, k.y);
-                            e = add_copies(e, d1.x, k.z);
-                            e = add_copies(e, d1.y, k.w);
+                    if (chunk <= COPIES) {   // the copies laid out one by one, zeros behind them
+                        const uint32_t at = static_cast<uint32_t>(upto - ns), n = static_cast<uint32_t>(chunk);
+                        for (uint32_t k = 0; k < ns; ++k) x[at + k] = static_cast<int>(lane) >= from ? ws : 0.0;
+                        if (lane < 8) x[n + lane] = 0.0;
+                        __syncwarp();
+                        const double2 *x2 = reinterpret_cast<const double2 *>(x);
+                        for (uint32_t i = 0; i < n; i += 8) {
+                            const double2 d0 = x2[i / 2], d1 = x2[i / 2 + 1], d2 = x2[i / 2 + 2], d3 = x2[i / 2 + 3];
+                            e += d0.x; e += d0.y; e += d1.x; e += d1.y;
+                            e += d2.x; e += d2.y; e += d3.x; e += d3.y;
                         }
+                    } else {
+                        for (int i = from; i < 32; ++i)
+                            e = add_repeated(e, __shfl_sync(FULL, ws, i), __shfl_sync(FULL, ns, i));
                     }
                     __syncwarp();
                 }
+                made += chunk;
             }
             if (static_cast<int>(lane) == l) {
                 ecell = e;
@@ -2620,6 +2686,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
                 if (in) {
                     pCount[q] = static_cast<uint32_t>(k - k0);
                     pWeight[q] = newEnergy;
+                    pOff[q] = static_cast<uint32_t>(k0);
                 }
             }
             if (static_cast<int>(lane) == l) m = static_cast<uint64_t>(before);
@@ -2639,8 +2706,8 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
 // 72^3 cells of which one in twenty holds a particle; 5.2 ms against 0.31 ms on 100
 // cells of 1700, 53 us against 18 us on 24^3 cells of 21).
 __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *W,
-                                   const double *Wtot, uint32_t *pCount, double *pWeight, uint64_t *cellCount,
-                                   double *eradCensus, DevStats *st) {
+                                   const double *Wtot, uint32_t *pCount, double *pWeight, uint32_t *pOff,
+                                   uint64_t *cellCount, double *eradCensus, DevStats *st) {
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -2663,11 +2730,13 @@ __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const 
                         for (uint64_t k = 0; k < ns; ++k) ecell += ws;
                         pCount[q] = static_cast<uint32_t>(ns);
                         pWeight[q] = ws;
+                        pOff[q] = static_cast<uint32_t>(m);
                         m += ns;
                     } else {
                         ecell += w;
                         pCount[q] = 1u | KEEP;
                         pWeight[q] = w;
+                        pOff[q] = static_cast<uint32_t>(m);
                         m += 1;
                     }
                 }
@@ -2684,6 +2753,7 @@ __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const 
                     cum += w;
                     pCount[q] = static_cast<uint32_t>(k - k0);
                     pWeight[q] = cc.e;
+                    pOff[q] = static_cast<uint32_t>(k0);
                 }
                 m = k;
             }
@@ -2692,8 +2762,7 @@ __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const 
         eradCensus[c] = ecell;
         eOut += ecell;
     }
-    eOut = warp_sum(eOut);
-    if ((threadIdx.x & 31) == 0 && eOut != 0.0) atomicAdd(&st->eCensusOut, eOut);
+    block_add(eOut, &st->eCensusOut);
 }
 
 // Exchange 2 of a sharded comb: every (shard, cell) run's weight and particle
@@ -2724,7 +2793,8 @@ __global__ void k_shard_cell_weights(const double *x, uint32_t ncells, uint32_t 
 // handle's part of each cell's census energy.
 __global__ void k_comb_plan_sharded(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *x,
                                     const double *Wc, const double *Wtot, uint32_t lo, uint32_t hi,
-                                    uint32_t *pCount, double *pWeight, double *eradCensus, DevStats *st) {
+                                    uint32_t *pCount, double *pWeight, uint32_t *pOff, uint64_t *runCount,
+                                    double *eradCensus, DevStats *st) {
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -2746,6 +2816,7 @@ __global__ void k_comb_plan_sharded(Ctx C, CombParams P, const double *wS, const
                 continue;
             }
             const uint32_t a = start[run], b = start[run + 1];
+            uint64_t m = 0;   // the run's copies
             if (none) {
                 for (uint32_t q = a; q < b; ++q) pCount[q] = 0;
             } else if (cc.mode == 0) {
@@ -2757,10 +2828,14 @@ __global__ void k_comb_plan_sharded(Ctx C, CombParams P, const double *wS, const
                         for (uint64_t k = 0; k < ns; ++k) ecell += ws;
                         pCount[q] = static_cast<uint32_t>(ns);
                         pWeight[q] = ws;
+                        pOff[q] = static_cast<uint32_t>(m);
+                        m += ns;
                     } else {
                         ecell += w;
                         pCount[q] = 1u | KEEP;
                         pWeight[q] = w;
+                        pOff[q] = static_cast<uint32_t>(m);
+                        m += 1;
                     }
                 }
             } else {
@@ -2776,9 +2851,12 @@ __global__ void k_comb_plan_sharded(Ctx C, CombParams P, const double *wS, const
                     cum += w;
                     pCount[q] = static_cast<uint32_t>(k - k0);
                     pWeight[q] = cc.e;
+                    pOff[q] = static_cast<uint32_t>(m);
+                    m += k - k0;
                 }
             }
             below += x[run];
+            runCount[run] = m;
         }
         eradCensus[c] = ecell;
         eOut += ecell;
@@ -2788,21 +2866,15 @@ __global__ void k_comb_plan_sharded(Ctx C, CombParams P, const double *wS, const
 }
 
 // Exchange 3 of a sharded comb: this handle's census particles per shard (the
-// copies its runs of shard s produce: the exclusive scan of the copy counts at
-// the shard's run boundaries) and its part of each cell's census energy.
-__global__ void k_shard_pack_census(const uint64_t *pOff, const uint64_t *total, const uint32_t *start, uint32_t n,
-                                    uint32_t ncells, uint32_t shards, uint32_t lo, uint32_t hi,
+// copies its runs of shard s produce: runOff, the exclusive scan of the runs'
+// copies, at the shard's run boundaries) and its part of each cell's census energy.
+__global__ void k_shard_pack_census(const uint64_t *runOff, uint32_t ncells, uint32_t shards, uint32_t lo, uint32_t hi,
                                     const double *eradCensus, double *x) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < shards) {
-        double v = 0.0;
-        if (t >= lo && t < hi) {
-            const uint32_t a = start[static_cast<size_t>(t) * ncells], b = start[static_cast<size_t>(t + 1) * ncells];
-            const uint64_t oa = a < n ? pOff[a] : *total, ob = b < n ? pOff[b] : *total;
-            v = static_cast<double>(ob - oa);
-        }
-        x[t] = v;
-    }
+    if (t < shards)
+        x[t] = t >= lo && t < hi ? static_cast<double>(runOff[static_cast<size_t>(t + 1) * ncells] -
+                                                       runOff[static_cast<size_t>(t) * ncells])
+                                 : 0.0;
     for (uint32_t c = t; c < ncells; c += gridDim.x * blockDim.x) x[shards + c] = eradCensus[c];
 }
 
@@ -2811,12 +2883,18 @@ __global__ void k_add_into(double *y, const double *x, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] += x[i];
 }
 
-// One thread per sorted particle writes its copies at its output offset.
-// The exclusive prefix of the copy counts over sorted particles is the output
-// position: cells are contiguous in sorted order and the output is cell-major.
-// Each thread takes EMIT_BATCH sorted particles per iteration and issues all
-// of their census-record gathers (read-only loads) before it writes any copy,
-// so the random reads overlap.
+// The output is in the order of the copies' groups (cells; sharded: (shard, cell)
+// runs) and within a group in sorted order: a particle's first copy goes to its
+// group's offset (the scan of the groups' copies) plus pOff.  Scanning the groups
+// instead of the particles saves four passes over the census.
+__device__ __forceinline__ uint64_t first_copy(const Ctx &C, uint64_t run, uint32_t bins, const uint64_t *groupOff,
+                                               uint32_t off) {
+    return groupOff[C.shards > 1 || bins == 1 ? run : run / bins] + off;
+}
+
+// One thread per sorted particle writes its copies.  Each thread takes EMIT_BATCH
+// sorted particles per iteration and issues all of their census-record gathers
+// (read-only loads) before it writes any copy, so the random reads overlap.
 constexpr int EMIT_BATCH = 2;
 
 // The copy of a census particle the comb writes (FP64 form): the new weight
@@ -2846,7 +2924,7 @@ __device__ __forceinline__ void comb_emit_fp64(const Ctx &C, PartReg &p, uint32_
 template <bool FP32>
 __global__ void k_comb_emit(Ctx C, CensusBank cen, const uint32_t *idx, const uint64_t *sortedKeys, int pidBits,
                             uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,
-                            const uint64_t *pOffset, Bank out) {
+                            const uint32_t *pOff, const uint64_t *groupOff, Bank out) {
     const uint32_t stride = gridDim.x * blockDim.x;
     constexpr int words = FP32 ? 4 : 6;
     for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < nValid; base += EMIT_BATCH * stride) {
@@ -2871,8 +2949,9 @@ __global__ void k_comb_emit(Ctx C, CensusBank cen, const uint32_t *idx, const ui
             const uint32_t m = raw[u] & ~KEEP;
             if (m == 0) continue;
             const uint32_t q = base + u * stride;
-            const uint32_t c = cell_of_run(C, sortedKeys[q] >> pidBits, bins);
-            const uint64_t o = pOffset[q];
+            const uint64_t run = sortedKeys[q] >> pidBits;
+            const uint32_t c = cell_of_run(C, run, bins);
+            const uint64_t o = first_copy(C, run, bins, groupOff, pOff[q]);
             const double wNew = pWeight[q];
             if constexpr (FP32) {
                 const uint4 a = rec[u][0], b = rec[u][1], d = rec[u][2];
@@ -2906,81 +2985,14 @@ __global__ void k_comb_emit(Ctx C, CensusBank cen, const uint32_t *idx, const ui
 // Output-driven form of the same write: one thread per output slot o, whose
 // source is the sorted particle src[o].  Every lane writes one particle, so
 // the bank writes are contiguous and no lane idles on a dropped particle.
-// src[o] comes from marking each particle with copies at its first slot and a
-// running maximum over the slots (the sources increase with the slots).
-__global__ void k_emit_src_mark(const uint32_t *pCount, const uint64_t *pOffset, uint32_t nValid, uint32_t *src) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nValid; q += gridDim.x * blockDim.x)
-        if (pCount[q] & ~KEEP) src[pOffset[q]] = q;
-}
-
-// inclusive running maximum of v[0, n) in tiles of 1024 (the tile's maximum to tileMax)
-__global__ void __launch_bounds__(1024) k_max_tiles(uint32_t *v, uint32_t n, uint32_t *tileMax) {
-    __shared__ uint32_t wmax[32];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t q = blockIdx.x * 1024u + threadIdx.x;
-    uint32_t x = q < n ? v[q] : 0u;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, x, d);
-        if (static_cast<int>(lane) >= d) x = max(x, y);
+__global__ void k_emit_src(Ctx C, const uint64_t *sortedKeys, int pidBits, uint32_t bins, const uint32_t *pCount,
+                           const uint32_t *pOff, const uint64_t *groupOff, uint32_t nValid, uint32_t *src) {
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nValid; q += gridDim.x * blockDim.x) {
+        const uint32_t n = pCount[q] & ~KEEP;
+        if (n == 0) continue;
+        const uint64_t o = first_copy(C, sortedKeys[q] >> pidBits, bins, groupOff, pOff[q]);
+        for (uint32_t k = 0; k < n; ++k) src[o + k] = q;
     }
-    if (lane == 31) wmax[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t w = wmax[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL, w, d);
-            if (static_cast<int>(lane) >= d) w = max(w, y);
-        }
-        wmax[lane] = w;
-    }
-    __syncthreads();
-    if (wid > 0) x = max(x, wmax[wid - 1]);
-    if (q < n) v[q] = x;
-    if (threadIdx.x == 1023) tileMax[blockIdx.x] = x;
-}
-// tileMax[t] <- maximum of tiles 0..t-1 (0 for t = 0), one block
-__global__ void __launch_bounds__(1024) k_max_tile_prefix(uint32_t *tileMax, uint32_t ntiles) {
-    __shared__ uint32_t wmax[32];
-    __shared__ uint32_t carryS;
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < ntiles; base += 1024u) {
-        const uint32_t q = base + threadIdx.x;
-        uint32_t x = q < ntiles ? tileMax[q] : 0u;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL, x, d);
-            if (static_cast<int>(lane) >= d) x = max(x, y);
-        }
-        if (lane == 31) wmax[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t w = wmax[lane];
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, w, d);
-                if (static_cast<int>(lane) >= d) w = max(w, y);
-            }
-            wmax[lane] = w;
-        }
-        __syncthreads();
-        if (wid > 0) x = max(x, wmax[wid - 1]);
-        const uint32_t incl = max(x, carry);
-        // exclusive: the inclusive maximum of the previous entry
-        uint32_t prev = __shfl_up_sync(FULL, incl, 1);
-        if (lane == 0) prev = wid > 0 ? max(wmax[wid - 1], carry) : carry;
-        if (q < ntiles) tileMax[q] = prev;
-        if (threadIdx.x == 1023) carryS = incl;
-        __syncthreads();
-        carry = carryS;
-        __syncthreads();
-    }
-}
-__global__ void __launch_bounds__(1024) k_max_apply(uint32_t *v, uint32_t n, const uint32_t *tileMax) {
-    const uint32_t q = blockIdx.x * 1024u + threadIdx.x;
-    if (q < n) v[q] = max(v[q], tileMax[blockIdx.x]);
 }
 
 template <bool FP32>
@@ -3110,7 +3122,8 @@ __global__ void k_strat_sums(const double *wS, const uint32_t *start, uint32_t n
 // sorted particles (bit 31 of the count: kept as is) and the census energy.
 __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *wS, const uint32_t *start,
                              const double *binW, const double *cellW, const double *Wtot, uint32_t *pCount,
-                             double *pWeight, uint64_t *cellCount, double *eradCensus, DevStats *st) {
+                             double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
+                             DevStats *st) {
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -3192,11 +3205,13 @@ __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *w
                             for (uint64_t k = 0; k < ns; ++k) ecell += ws;
                             pCount[q] = static_cast<uint32_t>(ns);
                             pWeight[q] = ws;
+                            pOff[q] = static_cast<uint32_t>(m);
                             m += ns;
                         } else {
                             ecell += w;
                             pCount[q] = 1u | KEEP;
                             pWeight[q] = w;
+                            pOff[q] = static_cast<uint32_t>(m);
                             m += 1;
                         }
                     }
@@ -3215,6 +3230,7 @@ __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *w
                         cum += w;
                         pCount[q] = static_cast<uint32_t>(k - k0);
                         pWeight[q] = newWeight;
+                        pOff[q] = static_cast<uint32_t>(m + k0);
                     }
                     m += k;
                 }
@@ -3226,13 +3242,6 @@ __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *w
     }
     eOut = warp_sum(eOut);
     if ((threadIdx.x & 31) == 0 && eOut != 0.0) atomicAdd(&st->eCensusOut, eOut);
-}
-
-// copies per sorted slot, over n slots of which the first *nValid are particles (zero beyond)
-__global__ void k_mask_count_upto(const uint32_t *pCount, uint32_t n, const uint32_t *nValid, uint64_t *out) {
-    const uint32_t v = *nValid;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
-        out[q] = q < v ? (pCount[q] & ~KEEP) : 0ull;
 }
 
 // census kept as is (no population control): order by pid for a deterministic bank
@@ -3465,7 +3474,12 @@ void launch_allocate_if(cudaStream_t s, const Ctx &C, const CellArrays &A, const
 void launch_emission_debit(cudaStream_t s, const Ctx &C, const CellArrays &A, DevStats *st) {
     k_emission_debit<<<grid_for(C.ncells, 256, 8192), 256, 0, s>>>(C, A, st);
 }
+uint32_t scan_launches(uint32_t n) { return n <= SCAN_ONE_BLOCK ? 1u : 3u; }
 void launch_scan_u64(cudaStream_t s, const uint64_t *in, uint32_t n, uint64_t *out, uint64_t *tileSums, uint64_t *total) {
+    if (n <= SCAN_ONE_BLOCK) {
+        k_scan_block<<<1, 1024, 0, s>>>(in, n, out, total);
+        return;
+    }
     const uint32_t tiles = (n + 1023) / 1024 ? (n + 1023) / 1024 : 1;
     k_scan_tiles<<<tiles, 1024, 0, s>>>(in, n, out, tileSums);
     k_scan_sums<<<1, 1024, 0, s>>>(tileSums, tiles, total);
@@ -3502,9 +3516,10 @@ void launch_strat_sums(cudaStream_t s, const double *wS, const uint32_t *start, 
 }
 void launch_strat_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const StratParams &S, const double *wS,
                        const uint32_t *start, const double *binW, const double *cellW, const double *Wtot,
-                       uint32_t *pCount, double *pWeight, uint64_t *cellCount, double *eradCensus, DevStats *st) {
+                       uint32_t *pCount, double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
+                       DevStats *st) {
     k_strat_plan<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, S, wS, start, binW, cellW, Wtot, pCount, pWeight,
-                                                             cellCount, eradCensus, st);
+                                                             pOff, cellCount, eradCensus, st);
 }
 void launch_transport(cudaStream_t s, uint32_t grid, const Ctx &C, const Bank &in, const uint32_t *nIn, const Bank &out,
                       uint32_t *nOut, const CensusBank &cen, uint32_t *nCen, uint32_t K, DevStats *st, int minBlocks) {
@@ -3587,20 +3602,25 @@ void launch_bucket_sort(cudaStream_t s, const Ctx &C, const CensusBank &cen, con
     cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), s);
     k_bucket_count<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(keys, n, pidBits, nRuns, start);
     const uint32_t stiles = (len + 1023) / 1024;
-    k_scan32_tiles<<<stiles, 1024, 0, s>>>(start, len, scanSums);
-    k_scan_sums<<<1, 1024, 0, s>>>(scanSums, stiles, scanSums + stiles);
-    k_scan32_add<<<stiles, 1024, 0, s>>>(start, len, scanSums);
+    if (len <= SCAN_ONE_BLOCK) {
+        k_scan32_block<<<1, 1024, 0, s>>>(start, len);
+    } else {
+        k_scan32_tiles<<<stiles, 1024, 0, s>>>(start, len, scanSums);
+        k_scan_sums<<<1, 1024, 0, s>>>(scanSums, stiles, scanSums + stiles);
+        k_scan32_add<<<stiles, 1024, 0, s>>>(start, len, scanSums);
+    }
     cudaMemcpyAsync(cursor, start, sizeof(uint32_t) * len, cudaMemcpyDeviceToDevice, s);
     k_bucket_place<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(keys, n, pidBits, nRuns, cursor, outKeys, outVals);
     k_bucket_sort_runs<<<grid_for(nRuns, BUCKET_WARPS, 148 * 32), 32 * BUCKET_WARPS, 0, s>>>(
-        C, cen, wc, outKeys, outVals, wS, start, nRuns, pidBits, longRuns, flags, longCap);
+        C, cen, wc, outKeys, outVals, wS, start, nRuns, pidBits, longRuns, flags, longCap,
+        nRuns < 4096u ? BUCKET_WARP_FEW : BUCKET_WARP_MAX);
     const size_t smem = sizeof(uint64_t) * BUCKET_BLOCK_MAX;
     cudaFuncSetAttribute(k_bucket_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    k_bucket_sort_long<<<148, 256, smem, s>>>(C, cen, wc, outKeys, outVals, wS, start, pidBits, longRuns, flags,
+    k_bucket_sort_long<<<148, BUCKET_LONG_THREADS, smem, s>>>(C, cen, wc, outKeys, outVals, wS, start, pidBits, longRuns, flags,
                                               longCap, flags + 1);
 }
 size_t bucket_scan_words(uint32_t len) { return (len + 1023) / 1024 + 2; }
-uint32_t bucket_long_capacity(uint32_t n) { return n / (BUCKET_WARP_MAX + 1) + 1; }
+uint32_t bucket_long_capacity(uint32_t n) { return n / (BUCKET_WARP_FEW + 1) + 1; }
 
 uint32_t radix_tile_count(uint32_t n) { return (n + RS_TILE - 1) / RS_TILE ? (n + RS_TILE - 1) / RS_TILE : 1; }
 // 32-bit words the radix sort needs for its tile histogram and the scan's tile sums
@@ -3629,48 +3649,40 @@ void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out
 }
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
-                      uint64_t *cellCount, double *eradCensus, DevStats *st) {
+                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st) {
     if (walk_by_thread(n, C.ncells)) {
         k_comb_plan_thread<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, wS, start, W, Wtot, pCount, pWeight,
-                                                                         cellCount, eradCensus, st);
+                                                                         pOff, cellCount, eradCensus, st);
         return;
     }
     k_comb_plan<<<walk_grid(C.ncells), 32 * WALK_WARPS, 0, s>>>(C, P, wS, start, W, upTo, Wtot, pCount, pWeight,
-                                                                cellCount, eradCensus, st, walk_batch(C.ncells));
+                                                                pOff, cellCount, eradCensus, st, walk_batch(C.ncells));
 }
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,
-                      const uint64_t *pOffset, const Bank &out) {
+                      const uint32_t *pOff, const uint64_t *groupOff, const Bank &out) {
     if (!nValid) return;
     if (C.fp32)
         k_comb_emit<true><<<grid_for(nValid, 256, 148 * 16), 256, 0, s>>>(C, cen, idx, sortedKeys, pidBits, bins, nValid, pCount,
-                                                                           pWeight, pOffset, out);
+                                                                           pWeight, pOff, groupOff, out);
     else
         k_comb_emit<false><<<grid_for(nValid, 256, 148 * 16), 256, 0, s>>>(C, cen, idx, sortedKeys, pidBits, bins, nValid, pCount,
-                                                                            pWeight, pOffset, out);
+                                                                            pWeight, pOff, groupOff, out);
 }
-// The same write, output-driven (k_comb_emit_out).  src: scratch of `total`
-// words; tileMax: scratch of total / 1024 + 1 words.
+// The same write, output-driven (k_comb_emit_out).  src: scratch of `total` words.
 void launch_comb_emit_out(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx,
                           const uint64_t *sortedKeys, int pidBits, uint32_t bins, uint32_t nValid, uint32_t total,
-                          const uint32_t *pCount, const double *pWeight, const uint64_t *pOffset, uint32_t *src,
-                          uint32_t *tileMax, const Bank &out) {
+                          const uint32_t *pCount, const double *pWeight, const uint32_t *pOff, const uint64_t *groupOff,
+                          uint32_t *src, const Bank &out) {
     if (!nValid || !total) return;
-    cudaMemsetAsync(src, 0, sizeof(uint32_t) * total, s);
-    k_emit_src_mark<<<grid_for(nValid, 256, 148 * 16), 256, 0, s>>>(pCount, pOffset, nValid, src);
-    const uint32_t tiles = (total + 1023) / 1024;
-    k_max_tiles<<<tiles, 1024, 0, s>>>(src, total, tileMax);
-    k_max_tile_prefix<<<1, 1024, 0, s>>>(tileMax, tiles);
-    k_max_apply<<<tiles, 1024, 0, s>>>(src, total, tileMax);
+    k_emit_src<<<grid_for(nValid, 256, 148 * 16), 256, 0, s>>>(C, sortedKeys, pidBits, bins, pCount, pOff, groupOff,
+                                                               nValid, src);
     if (C.fp32)
         k_comb_emit_out<true><<<grid_for(total, 256, 148 * 16), 256, 0, s>>>(C, cen, idx, sortedKeys, pidBits, bins, total,
                                                                              src, pCount, pWeight, out);
     else
         k_comb_emit_out<false><<<grid_for(total, 256, 148 * 16), 256, 0, s>>>(C, cen, idx, sortedKeys, pidBits, bins,
                                                                               total, src, pCount, pWeight, out);
-}
-void launch_mask_count_upto(cudaStream_t s, const uint32_t *pCount, uint32_t n, const uint32_t *nValid, uint64_t *out) {
-    k_mask_count_upto<<<grid_for(n, 256, 8192), 256, 0, s>>>(pCount, n, nValid, out);
 }
 void launch_census_keys_pid(cudaStream_t s, const Ctx &C, const CensusBank &cen, uint32_t n, uint64_t *keys,
                             uint32_t *vals) {
@@ -3760,10 +3772,15 @@ void launch_to_float(cudaStream_t s, const double *src, float *dst, uint32_t n) 
 }
 // Particles per cell at the start of transport (MonteCarloManagerSerial's
 // beginningParticleCount_, manager/MonteCarloManagerSerial.hpp:419-424).
+// Lanes of a warp with equal cells add once: the bank is in cell order (a
+// 100-cell slab of 2.7e5 particles took 140 us with an atomic per particle).
 __global__ void k_cell_histogram(const uint32_t *cell, uint32_t n, uint32_t N, uint32_t *count) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const uint32_t c = cell[q];
-        if (c < N) atomicAdd(count + c, 1u);
+    const unsigned lane = threadIdx.x & 31;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t q = base + threadIdx.x;
+        const uint32_t c = q < n ? cell[q] : 0xFFFFFFFFu;
+        const unsigned m = __match_any_sync(FULL, c);
+        if (c < N && static_cast<unsigned>(__ffs(m) - 1) == lane) atomicAdd(&count[c], static_cast<uint32_t>(__popc(m)));
     }
 }
 void launch_cell_histogram(cudaStream_t s, const uint32_t *cell, uint32_t n, uint32_t N, uint32_t *count) {
@@ -3777,17 +3794,15 @@ void launch_shard_cell_weights(cudaStream_t s, const double *x, uint32_t ncells,
 }
 void launch_comb_plan_sharded(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS,
                               const uint32_t *start, const double *x, const double *Wc, const double *Wtot,
-                              uint32_t lo, uint32_t hi, uint32_t *pCount, double *pWeight, double *eradCensus,
-                              DevStats *st) {
+                              uint32_t lo, uint32_t hi, uint32_t *pCount, double *pWeight, uint32_t *pOff,
+                              uint64_t *runCount, double *eradCensus, DevStats *st) {
     k_comb_plan_sharded<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, wS, start, x, Wc, Wtot, lo, hi, pCount,
-                                                                      pWeight, eradCensus, st);
+                                                                      pWeight, pOff, runCount, eradCensus, st);
 }
-void launch_shard_pack_census(cudaStream_t s, const uint64_t *pOff, const uint64_t *total, const uint32_t *start,
-                              uint32_t n, uint32_t ncells, uint32_t shards, uint32_t lo, uint32_t hi,
-                              const double *eradCensus, double *x) {
+void launch_shard_pack_census(cudaStream_t s, const uint64_t *runOff, uint32_t ncells, uint32_t shards, uint32_t lo,
+                              uint32_t hi, const double *eradCensus, double *x) {
     const uint32_t m = ncells > shards ? ncells : shards;
-    k_shard_pack_census<<<grid_for(m, 256, 8192), 256, 0, s>>>(pOff, total, start, n, ncells, shards, lo, hi,
-                                                                eradCensus, x);
+    k_shard_pack_census<<<grid_for(m, 256, 8192), 256, 0, s>>>(runOff, ncells, shards, lo, hi, eradCensus, x);
 }
 void launch_add_into(cudaStream_t s, double *y, const double *x, uint32_t n) {
     if (n) k_add_into<<<grid_for(n, 256, 8192), 256, 0, s>>>(y, x, n);

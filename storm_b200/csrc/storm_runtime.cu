@@ -101,8 +101,8 @@ struct StormHandle {
     size_t tileHistLen = 0;
     uint32_t *pCount = nullptr;      // comb: copies per sorted particle
     double *pWeight = nullptr;       // comb: weight of those copies
-    uint64_t *pOff = nullptr, *pTiles = nullptr;   // comb: output positions, scan tile sums
-    size_t restBytes = 0;            // the block holding bankC.rec through pTiles
+    double *pSum = nullptr;          // comb: compact census weights, then the running weights of the cells' sums
+    size_t restBytes = 0;            // the block holding bankC.rec through pSum
     // comb bucket sort scratch, grown on demand: run cursors and scan sums for
     // runLen runs, the list of long runs, and its two flags
     uint32_t *runCursor = nullptr, *longRuns = nullptr, *bucketFlags = nullptr;
@@ -113,7 +113,8 @@ struct StormHandle {
     uint64_t *offsets = nullptr, *tileSums = nullptr, *dTotalU64 = nullptr;
     double *dTotalE = nullptr, *combW = nullptr, *combWtot = nullptr;
     uint32_t *combStart = nullptr;
-    uint64_t *combCount = nullptr;
+    uint64_t *combCount = nullptr, *combOff = nullptr;     // copies per cell, and their scan (N + 1)
+    uint64_t *shardCount = nullptr, *shardOff = nullptr, *shardTiles = nullptr;   // the same per (shard, cell) run
     uint32_t *counts = nullptr;      // transport round counters (maxRounds + 1) + census counter
     DevStats *dStats = nullptr;
     int32_t *dErr = nullptr;
@@ -446,11 +447,10 @@ cudaError_t alloc_rest(StormHandle *h, size_t nc) {
                      reinterpret_cast<void **>(&h->keysAlt), reinterpret_cast<void **>(&h->vals),
                      reinterpret_cast<void **>(&h->valsAlt), reinterpret_cast<void **>(&h->tileHist),
                      reinterpret_cast<void **>(&h->pCount), reinterpret_cast<void **>(&h->pWeight),
-                     reinterpret_cast<void **>(&h->pOff), reinterpret_cast<void **>(&h->pTiles)};
+                     reinterpret_cast<void **>(&h->pSum)};
     const size_t bytes[] = {nc * census_words(h) * sizeof(uint4), nc * sizeof(uint64_t), nc * sizeof(uint64_t),
                             nc * sizeof(uint32_t), nc * sizeof(uint32_t), h->tileHistLen * sizeof(*h->tileHist),
-                            nc * sizeof(uint32_t), nc * sizeof(double), (nc + 1) * sizeof(uint64_t),
-                            (nc / 1024 + 4) * sizeof(uint64_t)};
+                            nc * sizeof(uint32_t), nc * sizeof(double), nc * sizeof(double)};
     size_t total = 0;
     for (size_t b : bytes) total += align256(b);
     unsigned char *base = nullptr;
@@ -458,7 +458,7 @@ cudaError_t alloc_rest(StormHandle *h, size_t nc) {
     if (e != cudaSuccess) return e;
     h->restBytes = total;
     size_t off = 0;
-    for (int q = 0; q < 10; ++q) {
+    for (int q = 0; q < 9; ++q) {
         *ptrs[q] = base + off;
         off += align256(bytes[q]);
     }
@@ -474,7 +474,7 @@ void free_rest(StormHandle *h, size_t) {
     h->tileHist = nullptr;
     h->pCount = nullptr;
     h->pWeight = nullptr;
-    h->pOff = h->pTiles = nullptr;
+    h->pSum = nullptr;
 }
 
 // (Re)allocate every per-particle buffer for capacity n, keeping the first
@@ -1157,6 +1157,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
         }
     }
     ALLOC(h->combCount, N + 1);
+    ALLOC(h->combOff, N + 1);
     h->maxRounds = d->max_rounds ? d->max_rounds : 16384;
     ALLOC(h->counts, h->maxRounds + 2);
     ALLOC(h->dStats, 1);
@@ -1356,12 +1357,12 @@ int storm_cuda_destroy(StormHandle *h) {
                   h->A.sigA, h->A.sigS, h->A.fleck, h->A.rwSigT, h->A.eradAvg, h->A.eradCensus, h->A.emitE,
                   h->A.rwElig, h->A.photons, h->A.phys, h->A.phys32, h->hx, h->hy, h->hz, h->segs, h->beginCounts, h->tabA, h->tabS, h->rhoF,
                   h->fsCell, h->fsSide, h->fsOffset, h->fsFace, h->fsArea, h->dAmbiguous, h->offsets, h->tileSums, h->dTotalU64, h->dTotalE, h->combW, h->combWtot,
-                  h->combStart, h->combCount, h->counts, h->dStats, h->dErr, h->gb, h->A.mgCdf, h->A.pgrw,
+                  h->combStart, h->combCount, h->combOff, h->counts, h->dStats, h->dErr, h->gb, h->A.mgCdf, h->A.pgrw,
                   h->A.pgrwCut, h->gb32, h->gc32, h->faceCdf, h->mgEp, h->mgEp32, h->mgKTq, h->ddmc, h->ddmcTot,
                   h->ddmcRate, h->ddmcCut, h->ddmc32, h->stratBounds, h->stratBinW, h->stratStart,
                   h->runCursor, h->runScan, h->longRuns, h->bucketFlags,
                   h->cfo, h->cfN, h->cfP, h->cfNext, h->cfFace, h->mpx, h->mpy, h->mpz, h->fvo, h->fvi, h->vtx,
-                  h->chord, h->cfN32, h->dep, h->att, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds,
+                  h->chord, h->cfN32, h->dep, h->att, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds, h->shardCount, h->shardOff, h->shardTiles,
                   h->vel, h->mom, h->ddmcCum32, h->cfA, h->egAvg, h->fixMat, h->fixRad, h->tetOff, h->tetCum,
                   h->tetAT};
     for (void *p : ps) device_pool().free(p);
@@ -1454,7 +1455,7 @@ static int emit_count(StormHandle *h, double dt, uint64_t *ne) {
     const double rel = 4.0 * (static_cast<double>(N) + 1100.0) * u;   // both orders' rounding, with margin
     launch_allocate_checked(h->stream, h->C, h->A, h->dTotalE, h->desc.new_photons_per_cell, rel, h->dAmbiguous);
     launch_scan_u64(h->stream, h->A.photons, N, h->offsets, h->tileSums, h->dTotalU64);
-    h->launches += 6;
+    h->launches += 3 + scan_launches(N);
     CK(cudaGetLastError());
     struct { uint64_t total; int32_t amb; } back{};
     {
@@ -1466,7 +1467,7 @@ static int emit_count(StormHandle *h, double dt, uint64_t *ne) {
         launch_sequential_sum(h->stream, h->A.emitE, N, h->dTotalE);
         launch_allocate(h->stream, h->C, h->A, h->dTotalE, h->desc.new_photons_per_cell);
         launch_scan_u64(h->stream, h->A.photons, N, h->offsets, h->tileSums, h->dTotalU64);
-        h->launches += 5;
+        h->launches += 2 + scan_launches(N);
         ++h->exactSums;
         CK(cudaGetLastError());
         CK(read_small(h, &back.total, h->dTotalU64, sizeof(uint64_t)));
@@ -1758,7 +1759,6 @@ static int comb_sharded(StormHandle *h) {
     P.ntotal = static_cast<uint64_t>(static_cast<double>(static_cast<uint64_t>(N) * h->desc.comb_nmin) * h->desc.comb_factor);
     if (n == 0) {
         CK(cudaMemsetAsync(start, 0, sizeof(uint32_t) * (R + 1), h->stream));
-        CK(cudaMemsetAsync(h->dTotalU64, 0, sizeof(uint64_t), h->stream));
     } else {
         launch_comb_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits);
         ++h->launches;
@@ -1782,7 +1782,7 @@ static int comb_sharded(StormHandle *h) {
             launch_bucket_sort(h->stream, h->C, h->bankC, h->keys, n, pidBits, static_cast<uint32_t>(R), start,
                                h->runCursor, h->runScan, h->keysAlt, h->valsAlt, wS, h->longRuns,
                                static_cast<uint32_t>(h->longCap), h->bucketFlags);
-            h->launches += 7;
+            h->launches += 4 + scan_launches(static_cast<uint32_t>(R) + 1);
             uint32_t flags[2] = {0, 0};
             const Readback r[1] = {{flags, h->bucketFlags, sizeof(flags)}};
             const int rc = read_many(h, r, 1, true);
@@ -1812,18 +1812,14 @@ static int comb_sharded(StormHandle *h) {
     if (rc != STORM_OK) return rc;
     launch_shard_cell_weights(h->stream, h->xbuf, N, S, h->shardWc);
     launch_blocked_sum(h->stream, h->shardWc, N, h->combWtot);
+    uint32_t *pOff = reinterpret_cast<uint32_t *>(skeys == h->keysAlt ? h->keys : h->keysAlt);   // the sort's spare key buffer
+    CK(cudaMemsetAsync(h->shardCount, 0, sizeof(uint64_t) * R, h->stream));   // the other ranks' runs hold nothing here
     launch_comb_plan_sharded(h->stream, h->C, P, wS, start, h->xbuf, h->shardWc, h->combWtot, h->shardLo,
-                             h->shardHi, h->pCount, h->pWeight, h->A.eradCensus, h->dStats);
-    h->launches += 3;
-    if (n) {
-        uint64_t *countU64 = skeys == h->keysAlt ? h->keys : h->keysAlt;   // the sort's spare key buffer
-        launch_mask_count_upto(h->stream, h->pCount, n, start + R, countU64);
-        launch_scan_u64(h->stream, countU64, n, h->pOff, h->pTiles, h->dTotalU64);
-        h->launches += 4;
-    }
+                             h->shardHi, h->pCount, h->pWeight, pOff, h->shardCount, h->A.eradCensus, h->dStats);
+    launch_scan_u64(h->stream, h->shardCount, static_cast<uint32_t>(R), h->shardOff, h->shardTiles, h->dTotalU64);
+    h->launches += 3 + scan_launches(static_cast<uint32_t>(R));
     // exchange 3: census particles per shard and census energy per cell
-    launch_shard_pack_census(h->stream, h->pOff, h->dTotalU64, start, n, N, S, h->shardLo, h->shardHi,
-                             h->A.eradCensus, h->xbuf);
+    launch_shard_pack_census(h->stream, h->shardOff, N, S, h->shardLo, h->shardHi, h->A.eradCensus, h->xbuf);
     ++h->launches;
     CK(cudaGetLastError());
     rc = exchange_sum(h, static_cast<uint64_t>(S) + N);
@@ -1850,14 +1846,14 @@ static int comb_sharded(StormHandle *h) {
         CK(bank_alloc(h, h->bankB, grown));
     }
     if (grown) {
-        launch_comb_emit(h->stream, h->C, h->bankC, idx, skeys, pidBits, 1, nValid, h->pCount, h->pWeight, h->pOff,
-                         h->bankA);
+        launch_comb_emit(h->stream, h->C, h->bankC, idx, skeys, pidBits, 1, nValid, h->pCount, h->pWeight, pOff,
+                         h->shardOff, h->bankA);
         ++h->launches;
     } else if (total) {
         uint32_t *src = idx == h->valsAlt ? h->vals : h->valsAlt;   // the sort's spare value buffer
         launch_comb_emit_out(h->stream, h->C, h->bankC, idx, skeys, pidBits, 1, nValid, static_cast<uint32_t>(total),
-                             h->pCount, h->pWeight, h->pOff, src, reinterpret_cast<uint32_t *>(h->pTiles), h->bankA);
-        h->launches += nValid ? 5 : 0;
+                             h->pCount, h->pWeight, pOff, h->shardOff, src, h->bankA);
+        h->launches += nValid ? 2 : 0;
     }
     CK(cudaGetLastError());
     if (grown) {
@@ -1911,9 +1907,8 @@ int storm_cuda_phase_comb(StormHandle *h) {
     const uint64_t nRuns = static_cast<uint64_t>(N) * B;
     uint32_t *start = strat ? h->stratStart : h->combStart;
     // the key kernel's compact copy of the census weights, for the bucket sort's
-    // sorted-weight gather; then the running weights of the cells' sums, for the
-    // plan; then the plan's output offsets
-    double *wc = reinterpret_cast<double *>(h->pOff), *upTo = wc;
+    // sorted-weight gather; then the running weights of the cells' sums, for the plan
+    double *wc = h->pSum, *upTo = h->pSum;
     if (strat) launch_strat_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, h->strat, wc);
     else launch_comb_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, wc);
     int cellBits = 0;
@@ -1926,6 +1921,7 @@ int storm_cuda_phase_comb(StormHandle *h) {
     // output total together, and only a failed bucket sort repeats the work.
     const uint64_t *skeys = nullptr;
     const uint32_t *idx = nullptr;
+    uint32_t *pOff = nullptr;  // a particle's first copy among its cell's: the sort's spare key buffer
     double *wS = h->pWeight;   // census weights in sorted order; the plan overwrites each slot with the copies' weight
     CombParams P;
     P.nmin = h->desc.comb_nmin;
@@ -1939,22 +1935,20 @@ int storm_cuda_phase_comb(StormHandle *h) {
         launch_sorted_weights(h->stream, h->C, h->bankC, idx, n, wS);
         h->launches += 5 * ((pidBits + cellBits + 7) / 8) + 2;
     };
-    // per-cell sums, the plan, and the copy counts scanned over n slots (the
-    // first start[nRuns] are particles, the rest count zero)
+    // per-cell sums, the plan, and the scan of the cells' copies
     auto plan_and_scan = [&]() {
+        pOff = reinterpret_cast<uint32_t *>(skeys == h->keysAlt ? h->keys : h->keysAlt);
         if (strat) launch_strat_sums(h->stream, wS, start, N, B, h->stratBinW, h->combW);
         else launch_comb_cell_sums(h->stream, wS, start, n, N, h->combW, upTo);
         launch_blocked_sum(h->stream, h->combW, N, h->combWtot);
         if (strat)
             launch_strat_plan(h->stream, h->C, P, h->strat, wS, start, h->stratBinW, h->combW, h->combWtot, h->pCount,
-                              h->pWeight, h->combCount, h->A.eradCensus, h->dStats);
+                              h->pWeight, pOff, h->combCount, h->A.eradCensus, h->dStats);
         else
             launch_comb_plan(h->stream, h->C, P, wS, start, n, h->combW, upTo, h->combWtot, h->pCount, h->pWeight,
-                             h->combCount, h->A.eradCensus, h->dStats);
-        uint64_t *countU64 = skeys == h->keysAlt ? h->keys : h->keysAlt;   // the sort's spare key buffer
-        launch_mask_count_upto(h->stream, h->pCount, n, start + nRuns, countU64);
-        launch_scan_u64(h->stream, countU64, n, h->pOff, h->pTiles, h->dTotalU64);
-        h->launches += 4 + 3;
+                             pOff, h->combCount, h->A.eradCensus, h->dStats);
+        launch_scan_u64(h->stream, h->combCount, N, h->combOff, h->tileSums, h->dTotalU64);
+        h->launches += 3 + scan_launches(N);
     };
     bool bucket = false;
     if (nRuns + 1 < 0xFFFFFFF0ull) {
@@ -1976,7 +1970,7 @@ int storm_cuda_phase_comb(StormHandle *h) {
         launch_bucket_sort(h->stream, h->C, h->bankC, h->keys, n, pidBits, static_cast<uint32_t>(nRuns), start,
                            h->runCursor, h->runScan, h->keysAlt, h->valsAlt, wS, h->longRuns,
                            static_cast<uint32_t>(h->longCap), h->bucketFlags, wc);
-        h->launches += 7;
+        h->launches += 4 + scan_launches(static_cast<uint32_t>(nRuns) + 1);
         skeys = h->keysAlt;
         idx = h->valsAlt;
         bucket = true;
@@ -1998,7 +1992,7 @@ int storm_cuda_phase_comb(StormHandle *h) {
         // a run too long for the bucket sort: sort by radix and plan again (the
         // plan adds the census energy to the step statistics, so that restarts)
         CK(cudaMemsetAsync(&h->dStats->eCensusOut, 0, sizeof(double), h->stream));
-        // the keys again: the first plan's copy counts went to their buffer
+        // the keys again: the first plan's copy offsets went to their buffer
         if (strat) launch_strat_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, h->strat);
         else launch_comb_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits);
         ++h->launches;
@@ -2024,14 +2018,14 @@ int storm_cuda_phase_comb(StormHandle *h) {
     }
     if (grown) {
         // the output-driven write needs `total` words of scratch, which only the grown buffers have
-        launch_comb_emit(h->stream, h->C, h->bankC, idx, skeys, pidBits, B, nValid, h->pCount, h->pWeight, h->pOff,
-                         h->bankA);
+        launch_comb_emit(h->stream, h->C, h->bankC, idx, skeys, pidBits, B, nValid, h->pCount, h->pWeight, pOff,
+                         h->combOff, h->bankA);
         ++h->launches;
     } else {
         uint32_t *src = idx == h->valsAlt ? h->vals : h->valsAlt;   // the sort's spare value buffer
         launch_comb_emit_out(h->stream, h->C, h->bankC, idx, skeys, pidBits, B, nValid, static_cast<uint32_t>(total),
-                             h->pCount, h->pWeight, h->pOff, src, reinterpret_cast<uint32_t *>(h->pTiles), h->bankA);
-        h->launches += nValid && total ? 5 : 0;
+                             h->pCount, h->pWeight, pOff, h->combOff, src, h->bankA);
+        h->launches += nValid && total ? 2 : 0;
     }
     CK(cudaGetLastError());
     if (grown) {
@@ -2108,6 +2102,9 @@ int storm_cuda_set_sharding(StormHandle *h, uint32_t shards, uint32_t lo, uint32
         CK(dalloc(h, &h->shardWc, N));
         CK(dalloc(h, &h->shardRunW, R));
         CK(dalloc(h, &h->shardStart, R + 2));
+        CK(dalloc(h, &h->shardCount, R));
+        CK(dalloc(h, &h->shardOff, R + 1));
+        CK(dalloc(h, &h->shardTiles, (R + 1023) / 1024 + 1));
         CK(dalloc(h, &h->shardBounds, 3 * (static_cast<size_t>(shards) + 1)));
         h->C.shardBounds = h->shardBounds;
     }
