@@ -28,6 +28,7 @@ struct CellArrays {
     double *T, *mass, *vol, *eint, *ceint;
     double *sigA, *sigS, *fleck, *rwSigT, *eradAvg, *eradCensus, *emitE;
     uint8_t *rwElig;
+    uint8_t *level;     // expected length of the histories that start here (history_level)
     uint64_t *photons;
     double4 *phys;      // per-cell segment constants (cell_phys)
     float4 *phys32;     // FP32-tracking form: 1/sigma_e, sigma_a f
@@ -56,6 +57,15 @@ struct FaceSources {
     const uint32_t *face;
     const double *area;
 };
+
+// The transport's queue: bank slots [first, end) in `chunks` chunks, taken in the
+// order of `order` (NULL: as they lie) at *next, which counts from zero.
+struct RefillQueue {
+    uint32_t first, end, chunk, chunks;
+    const uint32_t *order;
+    uint32_t *next;
+};
+constexpr uint32_t REFILL_CHUNK = 64;
 
 struct CombParams {
     uint64_t ntotal, nmin;
@@ -127,9 +137,12 @@ void launch_emit_faces(cudaStream_t s, const Ctx &C, const FaceSources &F, uint6
 void launch_transport(cudaStream_t s, uint32_t grid, const Ctx &C, const Bank &in, const uint32_t *nIn, const Bank &out,
                       uint32_t *nOut, const CensusBank &cen, uint32_t *nCen, uint32_t K, DevStats *st, int minBlocks);
 int transport_blocks_per_sm(int minBlocks, bool fp32);
-void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in, uint32_t n,
-                             uint32_t *nextIdx, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
+void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in,
+                             const RefillQueue &Q, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                              DevStats *st);
+// chunkLevel: Q.chunks bytes; counts: 32 words; order: Q.chunks words
+void launch_chunk_order(cudaStream_t s, const uint32_t *cell, const uint8_t *level, uint32_t n, const RefillQueue &Q,
+                        uint8_t *chunkLevel, uint32_t *counts, uint32_t *order);
 void launch_fold_attenuation(cudaStream_t s, const Ctx &C, DevStats *st);   // after the transport, where C.att is set
 int refill_blocks_per_sm(int minBlocks, bool fp32);
 void launch_bank_to_local(cudaStream_t s, const Ctx &C, const Bank &src, const Bank &dst, uint32_t n,
@@ -152,7 +165,8 @@ void launch_sorted_weights(cudaStream_t s, const Ctx &C, const CensusBank &cen, 
 // upTo: the running weight at each particle, NULL to leave it out
 void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *start, uint32_t n, uint32_t nRuns,
                            double *W, double *upTo = nullptr);
-void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out);
+// scratch: 1025 doubles, the last zero (NULL: one block sums)
+void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out, double *scratch = nullptr);
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
                       uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st);

@@ -447,6 +447,15 @@ __device__ inline void ddmc_cell_data(const Ctx &C, const CellArrays &A, uint32_
     if (C.ddmcCut) C.ddmcCut[c] = cutoff;
 }
 
+// Events a history can see in a step if it stays in the cell, as a power of two:
+// collisions over the step, or until absorption takes its weight below the cutoff
+// of 1e-3.  Orders the transport's chunks; nothing else depends on it.
+__device__ __forceinline__ uint8_t history_level(double sa, double ss, double f, double path) {
+    const double rate = ss + (1.0 - f) * sa, absorbed = f * sa;
+    const double events = rate * fmin(path, absorbed > 0.0 ? 6.9 / absorbed : path);
+    const int l = events > 1.0 ? ilogb(events) : 0;
+    return static_cast<uint8_t>(l > 15 ? 15 : l);
+}
 __global__ void k_prestep(Ctx C, CellArrays A, OpacityEos M, double dt) {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < C.ncells; c += gridDim.x * blockDim.x) {
         double sa, ss;
@@ -495,6 +504,7 @@ __global__ void k_prestep(Ctx C, CellArrays A, OpacityEos M, double dt) {
         if (f < 0.0 || f > 1.0) raise_error(C, STORM_DERR_FLECK, c, 0);
         A.phys[c] = cell_phys(sa, ss, f, sa + ss, C.clight);
         cell_rw_and_phys32(C, A, c, sa, ss, f);
+        A.level[c] = history_level(sa, ss, f, C.clight * dt);
         if (C.withDDMC) ddmc_cell_data(C, A, c, sa, ss);
     }
 }
@@ -1600,10 +1610,10 @@ __global__ void __launch_bounds__(256, MINB) k_transport32(Ctx C, Bank in, const
 // of `burst` segments.  The bank is in cell order, so a chunk of 64 keeps a
 // warp's cells together longer than one of 32 (64^3 gray cube: 5.85 to 5.69 ms
 // FP32, 20.2 to 19.6 ms FP64); longer ones leave a warp with a cell's long
-// histories at the end (256: 40^3 multigroup 1.0 to 1.5 ms), and the share shrinks
-// with what is left.  Per-lane totals live in the lane's own shared-memory slot
-// until the end, counts of ended histories in warp-uniform registers.  A history
-// longer than maxSegs raises STORM_DERR_HISTORY_CAP and stops.
+// histories at the end (256: 40^3 multigroup 1.0 to 1.5 ms).  Per-lane totals live
+// in the lane's own shared-memory slot until the end, counts of ended histories in
+// warp-uniform registers.  A history longer than maxSegs raises
+// STORM_DERR_HISTORY_CAP and stops.
 // What bounds it: instruction issue (77 % of the slots, 20 of 32 lanes, gray FP32)
 // or instruction fetch and divergence (FP64, multigroup), dependent loads of the
 // face planes on polyhedral meshes; a problem of few cells or few, long
@@ -1613,10 +1623,46 @@ __global__ void __launch_bounds__(256, MINB) k_transport32(Ctx C, Bank in, const
 // FP64 19.6 to 18.3; 24^3, 2.1e7 segments, FP32 0.78 to 0.50; 100-cell slab, 8e6
 // segments, FP64 3.1 to 1.4; 72^3 x 64 groups, 2.6e7 segments, FP32 2.77 to 1.90;
 // Voronoi 4e4 cells, 8.6e7 segments, FP32 6.4 to 6.2.
-constexpr uint32_t REFILL_CHUNK_MAX = 64;
+// A step of few histories ends with its longest one, so long ones are to start
+// first: the chunks are taken in the order of their cells' expected events
+// (history_level), cell order within a level.
+constexpr int LEVELS = 16;
+__global__ void k_chunk_levels(const uint32_t *cell, const uint8_t *level, uint32_t n, uint32_t chunk, uint32_t nChunks,
+                               uint8_t *chunkLevel, uint32_t *count) {
+    __shared__ uint32_t h[LEVELS];
+    if (threadIdx.x < LEVELS) h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < nChunks) {
+        const uint32_t a = k * chunk, b = min(a + chunk, n) - 1;
+        const uint8_t l = max(level[cell[a]], level[cell[b]]);
+        chunkLevel[k] = l;
+        atomicAdd(&h[l], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < LEVELS && h[threadIdx.x]) atomicAdd(&count[threadIdx.x], h[threadIdx.x]);
+}
+__global__ void k_chunk_order(const uint8_t *chunkLevel, uint32_t nChunks, const uint32_t *count, uint32_t *taken,
+                              uint32_t *order) {
+    __shared__ uint32_t h[LEVELS], base[LEVELS];
+    if (threadIdx.x < LEVELS) h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t at = 0;
+    const int l = k < nChunks ? chunkLevel[k] : 0;
+    if (k < nChunks) at = atomicAdd(&h[l], 1u);
+    __syncthreads();
+    if (threadIdx.x < LEVELS) {
+        uint32_t before = 0;   // the chunks of higher levels
+        for (int u = LEVELS - 1; u > static_cast<int>(threadIdx.x); --u) before += count[u];
+        base[threadIdx.x] = before + (h[threadIdx.x] ? atomicAdd(&taken[threadIdx.x], h[threadIdx.x]) : 0u);
+    }
+    __syncthreads();
+    if (k < nChunks) order[base[l] + at] = k;
+}
 
 template <class F, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, uint32_t n, uint32_t *nextIdx, CensusBank cen,
+__global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, RefillQueue Q, CensusBank cen,
                                                                  uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                                                                  DevStats *st) {
     __shared__ BlockStats bs;
@@ -1637,23 +1683,22 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
     uint32_t pid = 0, segsThis = 0;
     bool has = false;
     uint32_t cBase = 0, cLeft = 0;   // warp-uniform: this warp's chunk of unstarted particles
-    bool drained = false;            // warp-uniform: the bank counter has passed n
+    bool drained = false;            // warp-uniform: every chunk is taken
     uint32_t nEsc = 0, nCut = 0, nDone = 0;   // warp-uniform: histories ended so far, by outcome
     for (;;) {
         unsigned need = __ballot_sync(FULL, !has);
         while (need) {
             if (cLeft == 0) {
                 if (drained) break;
-                // a share of what was left at this warp's last chunk
-                const uint32_t share = (n - cBase) / (gridDim.x * 16u);
-                const uint32_t chunk = min(max(share & ~31u, 32u), REFILL_CHUNK_MAX);
-                uint32_t b = 0;
-                if (lane == 0) b = atomicAdd(nextIdx, chunk);
-                b = __shfl_sync(FULL, b, 0);
-                if (b >= n) { drained = true; break; }
-                if (n - b <= chunk) drained = true;
-                cBase = b;
-                cLeft = min(chunk, n - b);
+                uint32_t k = 0;
+                if (lane == 0) {
+                    k = atomicAdd(Q.next, 1u);
+                    if (k < Q.chunks && Q.order) k = Q.order[k];
+                }
+                k = __shfl_sync(FULL, k, 0);
+                if (k >= Q.chunks) { drained = true; break; }
+                cBase = Q.first + k * Q.chunk;
+                cLeft = min(Q.chunk, Q.end - cBase);
             }
             const uint32_t take = min(static_cast<uint32_t>(__popc(need)), cLeft);
             const uint32_t rank = __popc(need & lt);
@@ -2386,10 +2431,13 @@ constexpr uint32_t WALK_TILE = 256;
 constexpr int WALK_E = WALK_TILE / 32;
 static inline uint32_t walk_batch(uint32_t nRuns) {
     const uint32_t b = (nRuns + WALK_BLOCKS * WALK_WARPS - 1) / (WALK_BLOCKS * WALK_WARPS);
-    return b < 1 ? 1u : (b > 32 ? 32u : b);
+    return b < 1 ? 1u : (b > 8 ? 8u : b);
 }
-// a thread per run: enough runs to fill the chip, short on average
-static inline bool walk_by_thread(uint32_t n, uint32_t nRuns) { return nRuns >= 100000u && n / nRuns < 256u; }
+// A thread per run where there are runs enough to fill the chip and most are empty
+// or single (72^3 cells, 2e4 particles: sums 4.7 us and plan 15 us, by warps 14 and 63);
+// with 50 particles a run the warps are ahead (64^3 cells: sums 84 and plan 180 us, by
+// threads 38 and 421).
+static inline bool walk_by_thread(uint32_t n, uint32_t nRuns) { return nRuns >= 100000u && n / nRuns < 4u; }
 static inline uint32_t walk_grid(uint32_t nRuns) {
     const uint32_t perBlock = WALK_WARPS * walk_batch(nRuns);
     const uint32_t g = (nRuns + perBlock - 1) / perBlock;
@@ -2456,10 +2504,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_cell_sums(const double
     if (mine) W[c] = s;
 }
 
-// The same sums with a thread per run straight from memory: where there are runs
-// enough to fill the chip with a thread each and they are short, a warp's lines
-// stay in L1 while its lanes walk them, and nothing is staged (38 us against 50-99
-// us on 64^3 cells of 50 particles; 480 us against 43-80 on 100 cells of 1700).
+// The same sums with a thread per run straight from memory (walk_by_thread).
 __global__ void k_comb_cell_sums_thread(const double *wS, const uint32_t *start, uint32_t ncells, double *W) {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) {
         double s = 0.0;
@@ -2468,27 +2513,55 @@ __global__ void k_comb_cell_sums_thread(const double *wS, const uint32_t *start,
     }
 }
 
-// Deterministic total: thread t adds v[t], v[t + 1024], ... in order (coalesced),
-// then a pairwise tree over the 1024 partial sums.
-__global__ void k_blocked_sum(const double *v, uint32_t n, double *out) {
-    __shared__ double part[1024];
+// Deterministic total: partial sum t adds v[t], v[t + 1024], ... in order
+// (coalesced), then a pairwise tree over the 1024 partial sums.  Above
+// SUM_ONE_BLOCK values the partial sums are spread over SUM_BLOCKS blocks and the
+// last one to finish takes the tree (one block reads 2 MB in 22 us at 64^3 cells);
+// scratch: 1024 partial sums and a counter, zero before and after.
+constexpr uint32_t SUM_ONE_BLOCK = 16384, SUM_BLOCKS = 32;
+__device__ __forceinline__ double strided_sum(const double *v, uint32_t n, uint32_t t) {
     double s = 0.0;
-    uint32_t q = threadIdx.x;
-    for (; q + 7 * 1024 < n; q += 8 * 1024) {   // eight loads on their way at a time, added in order
-        double x[8];
+    uint32_t q = t;
+    for (; q < n && n - q > 15 * 1024; q += 16 * 1024) {   // sixteen loads on their way at a time, added in order
+        double x[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = v[q + u * 1024];
+        for (int u = 0; u < 16; ++u) x[u] = v[q + u * 1024];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s += x[u];
+        for (int u = 0; u < 16; ++u) s += x[u];
     }
     for (; q < n; q += 1024) s += v[q];
-    part[threadIdx.x] = s;
-    __syncthreads();
+    return s;
+}
+__device__ __forceinline__ void sum_tree(double *part, uint32_t threads, double *out) {
     for (uint32_t w = 512; w >= 1; w >>= 1) {
-        if (threadIdx.x < w) part[threadIdx.x] = part[threadIdx.x] + part[threadIdx.x + w];
         __syncthreads();
+        for (uint32_t t = threadIdx.x; t < w; t += threads) part[t] = part[t] + part[t + w];
     }
+    __syncthreads();
     if (threadIdx.x == 0) *out = part[0];
+}
+__global__ void __launch_bounds__(1024) k_blocked_sum(const double *v, uint32_t n, double *out) {
+    __shared__ double part[1024];
+    part[threadIdx.x] = strided_sum(v, n, threadIdx.x);
+    sum_tree(part, 1024, out);
+}
+__global__ void __launch_bounds__(1024 / SUM_BLOCKS) k_blocked_sum_wide(const double *v, uint32_t n, double *out,
+                                                                        double *scratch) {
+    constexpr uint32_t T = 1024 / SUM_BLOCKS;   // one warp
+    __shared__ double part[1024];
+    unsigned *done = reinterpret_cast<unsigned *>(scratch + 1024);
+    const uint32_t t = blockIdx.x * T + threadIdx.x;
+    __stcg(scratch + t, strided_sum(v, n, t));
+    __threadfence();
+    __syncwarp();
+    unsigned before = 0;
+    if (threadIdx.x == 0) before = atomicAdd(done, 1u);
+    before = __shfl_sync(FULL, before, 0);
+    if (before + 1 != SUM_BLOCKS) return;
+    __threadfence();
+    for (uint32_t i = threadIdx.x; i < 1024; i += T) part[i] = __ldcg(scratch + i);
+    sum_tree(part, T, out);
+    if (threadIdx.x == 0) *done = 0u;
 }
 
 struct CombCell {
@@ -2701,10 +2774,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
     if (lane == 0 && eOut != 0.0) atomicAdd(&st->eCensusOut, eOut);
 }
 
-// The same plan with a thread per cell, for runs as k_comb_cell_sums_thread takes
-// them (347 us against 415 us on 64^3 cells of 50 particles, 18 us against 72 us on
-// 72^3 cells of which one in twenty holds a particle; 5.2 ms against 0.31 ms on 100
-// cells of 1700, 53 us against 18 us on 24^3 cells of 21).
+// The same plan with a thread per cell (walk_by_thread).
 __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *W,
                                    const double *Wtot, uint32_t *pCount, double *pWeight, uint32_t *pOff,
                                    uint64_t *cellCount, double *eradCensus, DevStats *st) {
@@ -3644,8 +3714,9 @@ void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *sta
     }
     k_comb_cell_sums<<<walk_grid(nRuns), 32 * WALK_WARPS, 0, s>>>(wS, start, nRuns, W, upTo, walk_batch(nRuns));
 }
-void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out) {
-    k_blocked_sum<<<1, 1024, 0, s>>>(v, n, out);
+void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out, double *scratch) {
+    if (n <= SUM_ONE_BLOCK || !scratch) k_blocked_sum<<<1, 1024, 0, s>>>(v, n, out);
+    else k_blocked_sum_wide<<<SUM_BLOCKS, 1024 / SUM_BLOCKS, 0, s>>>(v, n, out, scratch);
 }
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
@@ -3693,53 +3764,60 @@ void launch_gather(cudaStream_t s, const Ctx &C, const CensusBank &src, const ui
     k_gather<<<grid_for(n, 256, 8192), 256, 0, s>>>(C, src, idx, n, dst, eradCensus, st);
 }
 template <class F>
-static void refill_launch(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in, uint32_t n,
-                          uint32_t *nextIdx, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
+static void refill_launch(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in,
+                          const RefillQueue &Q, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                           DevStats *st) {
     switch (minBlocks) {
-    case 4: k_transport_refill<F, 4><<<grid, 256, 0, s>>>(C, in, n, nextIdx, cen, nCen, burst, maxSegs, st); break;
-    case 3: k_transport_refill<F, 3><<<grid, 256, 0, s>>>(C, in, n, nextIdx, cen, nCen, burst, maxSegs, st); break;
-    case 2: k_transport_refill<F, 2><<<grid, 256, 0, s>>>(C, in, n, nextIdx, cen, nCen, burst, maxSegs, st); break;
-    default: k_transport_refill<F, 1><<<grid, 256, 0, s>>>(C, in, n, nextIdx, cen, nCen, burst, maxSegs, st); break;
+    case 4: k_transport_refill<F, 4><<<grid, 256, 0, s>>>(C, in, Q, cen, nCen, burst, maxSegs, st); break;
+    case 3: k_transport_refill<F, 3><<<grid, 256, 0, s>>>(C, in, Q, cen, nCen, burst, maxSegs, st); break;
+    case 2: k_transport_refill<F, 2><<<grid, 256, 0, s>>>(C, in, Q, cen, nCen, burst, maxSegs, st); break;
+    default: k_transport_refill<F, 1><<<grid, 256, 0, s>>>(C, in, Q, cen, nCen, burst, maxSegs, st); break;
     }
 }
-void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in, uint32_t n,
-                             uint32_t *nextIdx, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
+void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const Ctx &C, const Bank &in,
+                             const RefillQueue &Q, const CensusBank &cen, uint32_t *nCen, uint32_t burst, uint32_t maxSegs,
                              DevStats *st) {
     if (C.egAvg) {   // multigroup problems with the group time averages
-        if (C.fp32 && C.withDDMC) refill_launch<Form32MGEg>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32) refill_launch<Form32MGLeanEg>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.withHydro) refill_launch<Form64HydroEg>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.withDDMC) refill_launch<Form64FullEg>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else refill_launch<Form64MGEg>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
+        if (C.fp32 && C.withDDMC) refill_launch<Form32MGEg>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32) refill_launch<Form32MGLeanEg>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.withHydro) refill_launch<Form64HydroEg>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.withDDMC) refill_launch<Form64FullEg>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else refill_launch<Form64MGEg>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
         return;
     }
     if (C.fixMat) {   // reproducible tallies
-        if (C.fp32 && C.poly && C.withDDMC) refill_launch<Form32PolyDDMCFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32 && C.poly) refill_launch<Form32PolyFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32 && C.groups >= 2 && C.withDDMC) refill_launch<Form32MGFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32 && C.groups >= 2) refill_launch<Form32MGLeanFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32 && C.withDDMC) refill_launch<Form32Fix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.fp32) refill_launch<Form32LeanFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.poly && C.withDDMC) refill_launch<Form64PolyDDMCFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.poly) refill_launch<Form64PolyFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.groups >= 2 && !C.withDDMC) refill_launch<Form64MGFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else if (C.groups >= 2 || C.withDDMC) refill_launch<Form64FullFix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-        else refill_launch<Form64Fix>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
+        if (C.fp32 && C.poly && C.withDDMC) refill_launch<Form32PolyDDMCFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32 && C.poly) refill_launch<Form32PolyFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32 && C.groups >= 2 && C.withDDMC) refill_launch<Form32MGFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32 && C.groups >= 2) refill_launch<Form32MGLeanFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32 && C.withDDMC) refill_launch<Form32Fix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.fp32) refill_launch<Form32LeanFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.poly && C.withDDMC) refill_launch<Form64PolyDDMCFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.poly) refill_launch<Form64PolyFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.groups >= 2 && !C.withDDMC) refill_launch<Form64MGFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else if (C.groups >= 2 || C.withDDMC) refill_launch<Form64FullFix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+        else refill_launch<Form64Fix>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
         return;
     }
-    if (C.fp32 && C.poly && C.withDDMC) refill_launch<Form32PolyDDMC>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.fp32 && C.poly) refill_launch<Form32Poly>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.fp32 && C.groups >= 2 && C.withDDMC) refill_launch<Form32MG>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.fp32 && C.groups >= 2) refill_launch<Form32MGLean>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.fp32 && C.withDDMC) refill_launch<Form32>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.fp32) refill_launch<Form32Lean>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.poly && C.withDDMC) refill_launch<Form64PolyDDMC>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.poly) refill_launch<Form64Poly>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.withHydro) refill_launch<Form64Hydro>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.groups >= 2 && !C.withDDMC) refill_launch<Form64MG>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else if (C.groups >= 2 || C.withDDMC) refill_launch<Form64Full>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
-    else refill_launch<Form64>(s, grid, minBlocks, C, in, n, nextIdx, cen, nCen, burst, maxSegs, st);
+    if (C.fp32 && C.poly && C.withDDMC) refill_launch<Form32PolyDDMC>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.fp32 && C.poly) refill_launch<Form32Poly>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.fp32 && C.groups >= 2 && C.withDDMC) refill_launch<Form32MG>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.fp32 && C.groups >= 2) refill_launch<Form32MGLean>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.fp32 && C.withDDMC) refill_launch<Form32>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.fp32) refill_launch<Form32Lean>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.poly && C.withDDMC) refill_launch<Form64PolyDDMC>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.poly) refill_launch<Form64Poly>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.withHydro) refill_launch<Form64Hydro>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.groups >= 2 && !C.withDDMC) refill_launch<Form64MG>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else if (C.groups >= 2 || C.withDDMC) refill_launch<Form64Full>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+    else refill_launch<Form64>(s, grid, minBlocks, C, in, Q, cen, nCen, burst, maxSegs, st);
+}
+void launch_chunk_order(cudaStream_t s, const uint32_t *cell, const uint8_t *level, uint32_t n, const RefillQueue &Q,
+                        uint8_t *chunkLevel, uint32_t *counts, uint32_t *order) {
+    const uint32_t g = (Q.chunks + 255) / 256;
+    cudaMemsetAsync(counts, 0, 2 * LEVELS * sizeof(uint32_t), s);
+    k_chunk_levels<<<g, 256, 0, s>>>(cell, level, n, Q.chunk, Q.chunks, chunkLevel, counts);
+    k_chunk_order<<<g, 256, 0, s>>>(chunkLevel, Q.chunks, counts, counts + LEVELS, order);
 }
 void launch_fold_attenuation(cudaStream_t s, const Ctx &C, DevStats *st) {
     k_fold_attenuation<<<grid_for(C.ncells, 256, 8192), 256, 0, s>>>(C, st);

@@ -129,6 +129,8 @@ struct StormHandle {
     std::vector<uint64_t> shardCensus;   // census particles per shard after the last comb (every shard)
     uint64_t nCenGlobal = 0, nCellEmitGlobal = 0, nFaceEmitGlobal = 0;   // this step's global counts
     double *dep = nullptr;           // this handle's material deposits of the step (N)
+    double *sumScratch = nullptr;    // launch_blocked_sum (1025)
+    uint32_t *chunkCounts = nullptr; // launch_chunk_order (32)
     double *att = nullptr;           // gray problems: the transport's attenuation per cell (SegmentTallyRun)
     double4 *vel = nullptr;          // moving material: (vx, vy, vz, gamma) per cell
     double *egAvg = nullptr;         // group time averages (with_eg_time_avg): ncells x groups
@@ -983,7 +985,8 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     h->fp32 = d->precision == STORM_PRECISION_FP32_TRACK;
     // measured on B200 at 64^3: FP32 tracking fits 64 registers without spills (4 blocks of 256
     // per SM); the FP64 form is fastest at 80 registers (3 blocks)
-    h->minBlocks = h->fp32 ? 4 : 3;
+    // FP64 on polyhedral meshes: 4 (Voronoi 1.2e4 cells, 1.8e7 segments: 2.64 against 2.80 ms with 3)
+    h->minBlocks = h->fp32 || d->mesh ? 4 : 3;
     if (!poly) {
         std::vector<float> fx(d->nx), fy(d->ny), fz(d->nz);
         for (uint32_t i = 0; i < d->nx; ++i) fx[i] = static_cast<float>(0.5 * (h->hxe[i + 1] - h->hxe[i]));
@@ -1103,6 +1106,11 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     H2D(A.mass, d->mass, N);
     H2D(A.eint, d->internal_energy, N);
     H2D(A.ceint, d->cell_internal_energy ? d->cell_internal_energy : d->internal_energy, N);
+    ALLOC(h->sumScratch, 1025);
+    ZERO(h->sumScratch, 1025 * sizeof(double));
+    ALLOC(h->chunkCounts, 32);
+    ALLOC(A.level, N);
+    ZERO(A.level, N);
     if (d->groups < 2 && !d->with_hydro) {
         ALLOC(h->att, N);
         ZERO(h->att, N * sizeof(double));
@@ -1362,7 +1370,7 @@ int storm_cuda_destroy(StormHandle *h) {
                   h->ddmcRate, h->ddmcCut, h->ddmc32, h->stratBounds, h->stratBinW, h->stratStart,
                   h->runCursor, h->runScan, h->longRuns, h->bucketFlags,
                   h->cfo, h->cfN, h->cfP, h->cfNext, h->cfFace, h->mpx, h->mpy, h->mpz, h->fvo, h->fvi, h->vtx,
-                  h->chord, h->cfN32, h->dep, h->att, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds, h->shardCount, h->shardOff, h->shardTiles,
+                  h->chord, h->cfN32, h->dep, h->att, h->sumScratch, h->chunkCounts, h->A.level, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds, h->shardCount, h->shardOff, h->shardTiles,
                   h->vel, h->mom, h->ddmcCum32, h->cfA, h->egAvg, h->fixMat, h->fixRad, h->tetOff, h->tetCum,
                   h->tetAT};
     for (void *p : ps) device_pool().free(p);
@@ -1449,7 +1457,7 @@ static int emit_count(StormHandle *h, double dt, uint64_t *ne) {
     // settles almost every step; a flagged step recomputes with the exact
     // left-to-right total.  Either way the counts equal the reference's.
     launch_emission_energy(h->stream, h->C, h->A, dt);
-    launch_blocked_sum(h->stream, h->A.emitE, N, h->dTotalE);
+    launch_blocked_sum(h->stream, h->A.emitE, N, h->dTotalE, h->sumScratch);
     CK(cudaMemsetAsync(h->dAmbiguous, 0, sizeof(int32_t), h->stream));
     const double u = 0x1p-53;
     const double rel = 4.0 * (static_cast<double>(N) + 1100.0) * u;   // both orders' rounding, with margin
@@ -1565,6 +1573,16 @@ static int exchange_tallies(StormHandle *h) {
     return STORM_OK;
 }
 
+// The transport's queue over bank slots [first, end); its counter is h->counts[1],
+// set to zero before.  A chunk is a warp's 32 lanes while the bank is a few times
+// what the chip takes at once, so that no warp holds particles back from idle lanes.
+static RefillQueue refill_queue(StormHandle *h, uint64_t first, uint64_t end) {
+    const uint32_t len = static_cast<uint32_t>(end - first);
+    const uint32_t chunk = len > 8ull * 1024 * static_cast<uint64_t>(h->smCount) ? REFILL_CHUNK : 32u;
+    return RefillQueue{static_cast<uint32_t>(first), static_cast<uint32_t>(end), chunk, (len + chunk - 1) / chunk, nullptr,
+                       h->counts + 1};
+}
+
 int storm_cuda_phase_transport(StormHandle *h) {
     if (!h) return STORM_ERR_INVALID_ARG;
     refresh_ctx(h);
@@ -1623,9 +1641,23 @@ int storm_cuda_phase_transport(StormHandle *h) {
                 h->evPool.resize(8);
                 for (auto &e : h->evPool) CK(cudaEventCreate(&e));
             }
+            RefillQueue Q = refill_queue(h, 0, n32);
+            // Long histories first, where the bank is up to eight times what starts at
+            // once: Densmore slab, 5.2e5 histories, 10.6 to 8.5 ms; 24^3 cube, 6.7e5, 0.49
+            // to 0.46; 100-cell slab, 2.7e5, 1.31 to 1.34.  Larger banks end evenly
+            // anyway and lose their cell order (72^3 multigroup, 9.4e6: 1.81 to 1.89).
+            const uint64_t atOnce = static_cast<uint64_t>(grid) * 256;
+            if (n0 > atOnce && n0 <= 8 * atOnce) {
+                // the comb's sort buffers are idle during the transport
+                uint32_t *order = h->vals;
+                launch_chunk_order(h->stream, h->bankA.cell, h->A.level, n32, Q, reinterpret_cast<uint8_t *>(h->valsAlt),
+                                   h->chunkCounts, order);
+                Q.order = order;
+                h->launches += 2;
+            }
             if (h->profiling) CK(cudaEventRecord(h->evPool[0], h->stream));
-            launch_transport_refill(h->stream, grid, h->minBlocks, h->C, h->bankA, n32, h->counts + 1, h->bankC, nCen,
-                                    h->burst, maxSegs, h->dStats);
+            launch_transport_refill(h->stream, grid, h->minBlocks, h->C, h->bankA, Q, h->bankC, nCen, h->burst, maxSegs,
+                                    h->dStats);
             if (h->profiling) CK(cudaEventRecord(h->evPool[1], h->stream));
             ++h->launches;
             if (h->att) {
@@ -1811,7 +1843,7 @@ static int comb_sharded(StormHandle *h) {
     int rc = exchange_sum(h, 2 * R);
     if (rc != STORM_OK) return rc;
     launch_shard_cell_weights(h->stream, h->xbuf, N, S, h->shardWc);
-    launch_blocked_sum(h->stream, h->shardWc, N, h->combWtot);
+    launch_blocked_sum(h->stream, h->shardWc, N, h->combWtot, h->sumScratch);
     uint32_t *pOff = reinterpret_cast<uint32_t *>(skeys == h->keysAlt ? h->keys : h->keysAlt);   // the sort's spare key buffer
     CK(cudaMemsetAsync(h->shardCount, 0, sizeof(uint64_t) * R, h->stream));   // the other ranks' runs hold nothing here
     launch_comb_plan_sharded(h->stream, h->C, P, wS, start, h->xbuf, h->shardWc, h->combWtot, h->shardLo,
@@ -1940,7 +1972,7 @@ int storm_cuda_phase_comb(StormHandle *h) {
         pOff = reinterpret_cast<uint32_t *>(skeys == h->keysAlt ? h->keys : h->keysAlt);
         if (strat) launch_strat_sums(h->stream, wS, start, N, B, h->stratBinW, h->combW);
         else launch_comb_cell_sums(h->stream, wS, start, n, N, h->combW, upTo);
-        launch_blocked_sum(h->stream, h->combW, N, h->combWtot);
+        launch_blocked_sum(h->stream, h->combW, N, h->combWtot, h->sumScratch);
         if (strat)
             launch_strat_plan(h->stream, h->C, P, h->strat, wS, start, h->stratBinW, h->combW, h->combWtot, h->pCount,
                               h->pWeight, pOff, h->combCount, h->A.eradCensus, h->dStats);
@@ -2255,10 +2287,10 @@ static int step_host_overlapped(StormHandle *h, double dt, const StormParticlesS
         return need < g ? (need ? need : 1u) : g;
     };
     if (nb > n) {
-        launch_set_u32(h->stream, h->counts + 1, static_cast<uint32_t>(n));   // the refill queue starts at n
         launch_transport_refill(h->stream, grid_for_range(nb - n), h->minBlocks, h->C, h->bankA,
-                                static_cast<uint32_t>(nb), h->counts + 1, h->bankC, nCen, h->burst, maxSegs, h->dStats);
-        h->launches += 2;
+                                refill_queue(h, n, nb), h->bankC, nCen,
+                                h->burst, maxSegs, h->dStats);
+        ++h->launches;
     }
     // the rest of the census behind the work above (from pageable memory the host
     // itself copies while the device runs that work), in chunks that each join
@@ -2293,10 +2325,10 @@ static int step_host_overlapped(StormHandle *h, double dt, const StormParticlesS
             launch_cell_histogram(h->stream, h->bankA.cell, static_cast<uint32_t>(nb), h->N, h->beginCounts);
             ++h->launches;
         }
-        launch_set_u32(h->stream, h->counts + 1, static_cast<uint32_t>(lo));
+        launch_set_u32(h->stream, h->counts + 1, 0u);   // the queue's counter
         launch_transport_refill(h->stream, grid_for_range(hi - lo), h->minBlocks, h->C, h->bankA,
-                                static_cast<uint32_t>(hi), h->counts + 1, h->bankC, nCen, h->burst, maxSegs,
-                                h->dStats);
+                                refill_queue(h, lo, hi), h->bankC, nCen,
+                                h->burst, maxSegs, h->dStats);
         h->launches += 2;
     }
     if (h->att) {
