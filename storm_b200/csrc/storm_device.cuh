@@ -21,10 +21,12 @@ namespace storm {
 enum : int { NO_CELL_MOVE = 0, CELL_MOVE = 1, DONE = 2, REMOVE = 3, REFLECT = 4 };
 // a scatter whose new direction (and frequency) the caller still draws (finish64)
 enum : int { SCATTER = 5, SCATTER_EFFECTIVE = 6 };
+enum : int { JUMP = 7 };   // a Random Walk jump that the caller takes later (jump64)
 // outcome of a segment after the manager's handling
 enum : int { OUT_CONTINUE = 0, OUT_CENSUS = 1, OUT_CUTOFF = 2, OUT_ESCAPE = 3, OUT_ERROR = -1 };
 // left by a segment of the persistent transport for its finish (finish64, finish32)
 enum : int { OUT_SCATTER = 4, OUT_REEMIT = 5 };
+enum : int { OUT_JUMP = 6 };   // a Random Walk jump for the end of the burst (jump64, jump32)
 // random stream tags
 enum : uint32_t { TAG_TRANSPORT = 1, TAG_CELL_EMIT = 2, TAG_FACE_EMIT = 3, TAG_COMB = 4 };
 
@@ -1230,7 +1232,37 @@ __device__ __forceinline__ void track_begin(const Ctx &C, Track &T) {
 // V = 2 is the convex-polyhedral form: the face search of
 // distanceToNearestFace over the cell's inward normals and face centroids as
 // written (alpha = ((faceCM - x).n) / (n.v), the first smallest positive).
-// LATER leaves a scatter to finish64 (status SCATTER or SCATTER_EFFECTIVE).
+// LATER leaves a scatter to finish64 (status SCATTER or SCATTER_EFFECTIVE) and, in
+// the gray forms, a Random Walk jump to jump64 (status JUMP).
+
+// Whether try_random_walk takes the jump (gray): its own test
+template <class GEOM>
+__device__ __forceinline__ bool rw_wanted(const Ctx &C, const PartReg &p, const double4 &cp, const GEOM &g) {
+    double Ro = DBL_MAX;
+    for (int s = 0; s < g.nf(); ++s) {
+        const double d = g.dist(s, p.x, p.y, p.z);
+        Ro = (d < Ro) ? d : Ro;
+    }
+    Ro = (Ro > 0.0) ? Ro : 0.0;
+    const double sigmaT = C.rwSigT[p.cell];
+    return Ro > 0.0 && sigmaT > 0.0 && cp.w > 0.0 && Ro * sigmaT >= C.rwMinParticle;
+}
+__device__ __forceinline__ CartGeom cart_geom(const Ctx &C, uint32_t i, uint32_t j, uint32_t k) {
+    return CartGeom{C.xe[i], C.xe[i + 1], C.ye[j], C.ye[j + 1], C.ze[k], C.ze[k + 1], C.xc[i], C.yc[j], C.zc[k]};
+}
+__device__ __forceinline__ PolyGeom poly_geom(const Ctx &C, uint32_t cell) {
+    return PolyGeom{&C, C.cfo[cell], C.cfo[cell + 1], C.mpx[cell], C.mpy[cell], C.mpz[cell]};
+}
+// The jump that a segment left (gray): the ParticleStatus, or -2 where the shrink loop gives up
+template <bool POLY, class RNG, class TALLY>
+__device__ inline int jump64(const Ctx &C, Track &T, RNG &rng, TALLY &tal) {
+    const double4 cp = C.phys[T.p.cell];
+    int r;
+    if constexpr (POLY) r = try_random_walk<false>(C, T.p, rng, tal, cp, poly_geom(C, T.p.cell));
+    else r = try_random_walk<false>(C, T.p, rng, tal, cp, cart_geom(C, T.i, T.j, T.k));
+    T.speed = vnorm(T.p.vx, T.p.vy, T.p.vz);
+    return r;
+}
 
 // The end of a scatter: the isotropic direction and, in a multigroup problem,
 // the clamped or re-emitted frequency (:1826-1852).  False where the spectrum
@@ -1346,13 +1378,19 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
     }
 
     if (C.withRW && C.rwElig[cell]) {
-        int r;
-        if constexpr (POLY) {
-            const PolyGeom g{&C, C.cfo[cell], C.cfo[cell + 1], C.mpx[cell], C.mpy[cell], C.mpz[cell]};
-            r = try_random_walk<FULL>(C, p, rng, tal, cp, g);
+        int r = -1;
+        if constexpr (LATER && !FULL) {
+            bool wanted;
+            if constexpr (POLY) wanted = rw_wanted(C, p, cp, poly_geom(C, cell));
+            else wanted = rw_wanted(C, p, cp, cart_geom(C, i, j, k));
+            if (wanted) {
+                o.status = JUMP;
+                return o;
+            }
+        } else if constexpr (POLY) {
+            r = try_random_walk<FULL>(C, p, rng, tal, cp, poly_geom(C, cell));
         } else {
-            const CartGeom g{C.xe[i], C.xe[i + 1], C.ye[j], C.ye[j + 1], C.ze[k], C.ze[k + 1], C.xc[i], C.yc[j], C.zc[k]};
-            r = try_random_walk<FULL, CartGeom, RNG, TALLY, HYDRO>(C, p, rng, tal, cp, g);
+            r = try_random_walk<FULL, CartGeom, RNG, TALLY, HYDRO>(C, p, rng, tal, cp, cart_geom(C, i, j, k));
         }
         if (r == -2) { o.errCode = STORM_DERR_RW_SHRINK; return o; }
         if (r >= 0) {
@@ -1851,7 +1889,26 @@ __device__ __forceinline__ bool finish32(const Ctx &C, Track32 &T, RNG &rng, boo
     return true;
 }
 
-template <bool MG, bool LATER, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
+// the particle's distance to its cell's nearest face
+template <bool POLY>
+__device__ __forceinline__ float nearest_face32(const Ctx &C, const Track32 &T) {
+    if constexpr (POLY) {
+        float Ro = FLT_MAX;
+#pragma unroll 4
+        for (uint32_t k = C.cfo[T.cell]; k < C.cfo[T.cell + 1]; ++k) Ro = fminf(Ro, poly_dist32(C, k, T.qx, T.qy, T.qz));
+        return Ro;
+    } else {
+        return fminf(fminf(T.hx - fabsf(T.qx), T.hy - fabsf(T.qy)), T.hz - fabsf(T.qz));
+    }
+}
+// The Random Walk jump that a segment left (OUT_JUMP), gray
+template <bool POLY, class RNG, class TALLY>
+__device__ inline int jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, int &err) {
+    return rw_jump32<false, POLY>(C, T, rng, tal, T.cp, nearest_face32<POLY>(C, T), T.hx, T.hy, T.hz, err);
+}
+
+// JUMPS leaves a Random Walk jump (OUT_JUMP) to jump32.
+template <bool MG, bool LATER, bool JUMPS, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
 __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, int &usedRW, int &err) {
     const uint32_t cell = T.cell;
     // the draws a segment can take: the collision and the scatter's two; in a
@@ -1871,15 +1928,12 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         // only Random Walk and DDMC cells (finite reach) need the distance to the faces
         Ro = 0.0f;
         const bool ddmcCell = DDMC && C.withDDMC && C.ddmc32[3 * static_cast<size_t>(cell)].x < CUDART_INF_F;
-        if (cp.z < CUDART_INF_F || ddmcCell) {
-            Ro = FLT_MAX;
-#pragma unroll 4
-            for (uint32_t k = C.cfo[cell]; k < C.cfo[cell + 1]; ++k) Ro = fminf(Ro, poly_dist32(C, k, T.qx, T.qy, T.qz));
-        }
+        if (cp.z < CUDART_INF_F || ddmcCell) Ro = nearest_face32<true>(C, T);
     } else {
-        Ro = fminf(fminf(hx - fabsf(T.qx), hy - fabsf(T.qy)), hz - fabsf(T.qz));
+        Ro = nearest_face32<false>(C, T);
     }
     if (Ro >= cp.z && Ro > 0.0f && (!MG || static_cast<double>(T.nu) < C.gb[C.pgrwCut[cell]])) {
+        if constexpr (JUMPS) return OUT_JUMP;
         usedRW = 1;
         return rw_jump32<MG, POLY>(C, T, rng, tal, cp, Ro, hx, hy, hz, err);
     }
@@ -2112,6 +2166,7 @@ __device__ __forceinline__ int manager_handle(const Ctx &C, Track &T, const Phys
     if (o.status == DONE) return OUT_CENSUS;
     if (o.status == SCATTER) return OUT_SCATTER;
     if (o.status == SCATTER_EFFECTIVE) return OUT_REEMIT;
+    if (o.status == JUMP) return OUT_JUMP;
     return OUT_CONTINUE;
 }
 

@@ -1397,6 +1397,7 @@ __device__ __forceinline__ void block_stats_flush(const BlockStats &bs, DevStats
 template <int V, class TL = SegmentTally>
 struct Form64T {
     static constexpr bool kTogether = true;
+    static constexpr bool kJumpsLater = V == 0 || V == 2 || V == 5;   // gray
     using T = Track;
     using Rng = PhiloxRng;       // bank visits
     using Ring = PhiloxRing2;    // the persistent transport
@@ -1412,7 +1413,7 @@ struct Form64T {
                                                  uint32_t draw) {
         census_store64(b, q, t.p, pid, draw);
     }
-    template <bool LATER, class RNG, class TALLY>
+    template <bool LATER, bool JUMPS, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
         PhysOut o = physics_step<V, LATER>(C, t, rng, tal);
         if (o.errCode) { err = o.errCode; return OUT_ERROR; }
@@ -1426,6 +1427,13 @@ struct Form64T {
     template <class RNG>
     static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int left) {
         return finish64<V == 1 || V == 4>(C, t, rng, left == OUT_REEMIT);
+    }
+    // the Random Walk jump a segment left (OUT_JUMP)
+    template <class RNG, class TALLY>
+    static __device__ __forceinline__ int jump(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &err) {
+        const int r = jump64<V == 2 || V == 5>(C, t, rng, tal);
+        if (r == -2) { err = STORM_DERR_RW_SHRINK; return OUT_ERROR; }
+        return r == REMOVE ? OUT_CUTOFF : (r == DONE ? OUT_CENSUS : OUT_CONTINUE);
     }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.p.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.p.w; }
@@ -1447,6 +1455,7 @@ using Form64PolyDDMCFix = Form64T<5, SegmentTallyFixed>;
 template <bool POLY, bool DDMC = true, class TL = SegmentTally>
 struct Form32T {
     static constexpr bool kTogether = POLY;
+    static constexpr bool kJumpsLater = false;   // 64^3 5.7 to 5.8 ms, 24^3 0.47 to 0.49, served problems 75 to 72
     using T = Track32;
     using Rng = PhiloxRng4;      // bank visits
     using Ring = PhiloxRing4;    // the persistent transport
@@ -1462,15 +1471,19 @@ struct Form32T {
                                                  uint32_t draw) {
         census_store32(b, q, t, pid, draw);
     }
-    template <bool LATER, class RNG, class TALLY>
+    template <bool LATER, bool JUMPS, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<false, LATER, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<false, LATER, JUMPS, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
         return m;
     }
     template <class RNG>
     static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int) {
         return finish32<false>(C, t, rng, true);
+    }
+    template <class RNG, class TALLY>
+    static __device__ __forceinline__ int jump(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &err) {
+        return jump32<POLY>(C, t, rng, tal, err);
     }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.w; }
@@ -1487,6 +1500,7 @@ using Form32PolyDDMCFix = Form32T<true, true, SegmentTallyFixed>;
 template <bool DDMC = true, class TL = SegmentTally>
 struct Form32MGT {
     static constexpr bool kTogether = true;
+    static constexpr bool kJumpsLater = false;   // every other segment is a jump
     using T = Track32;
     using Rng = PhiloxRng4;      // bank visits
     using Ring = PhiloxRing4;    // the persistent transport
@@ -1504,9 +1518,9 @@ struct Form32MGT {
                                                  uint32_t draw) {
         census_store32_mg(b, q, t, pid, draw);
     }
-    template <bool LATER, class RNG, class TALLY>
+    template <bool LATER, bool JUMPS, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<true, LATER, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<true, LATER, false, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
         if (m == OUT_CONTINUE && t.nu < 0.0f) m = OUT_REEMIT;   // a Random Walk's upscatter
         return m;
@@ -1552,7 +1566,7 @@ __device__ __forceinline__ void visit_bank(const Ctx &C, const Bank &in, uint32_
                 tal.enter(cell0);
                 ++s;
                 int usedRW = 0, err = 0;
-                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false, false>(C, t, rng, tal, usedRW, err);
                 rw += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
@@ -1737,9 +1751,9 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                     tal.enter(cell0);
                     ++segsThis;
                     int usedRW = 0, err = 0;
-                    outcome = F::template seg<true>(C, t, rng, tal, usedRW, err);
+                    outcome = F::template seg<true, F::kJumpsLater>(C, t, rng, tal, usedRW, err);
                     rws += usedRW;
-                    if (outcome >= OUT_SCATTER) {
+                    if (outcome == OUT_SCATTER || outcome == OUT_REEMIT) {
                         left = outcome;
                         outcome = OUT_CONTINUE;
                     }
@@ -1765,7 +1779,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                 tal.enter(cell0);
                 ++segsThis;
                 int usedRW = 0, err = 0;
-                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false, F::kJumpsLater>(C, t, rng, tal, usedRW, err);
                 rws += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
@@ -1775,6 +1789,25 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                     raise_error(C, STORM_DERR_HISTORY_CAP, cell0, pid);
                     outcome = OUT_ERROR;
                     break;
+                }
+            }
+        }
+        // In the gray FP64 forms a Random Walk jump ends its lane's burst, and the lanes
+        // that came to one take it here together.  The jump's code is longer than the
+        // segment's, and the instruction cache serves the burst's loop better without
+        // it (64^3 cube 18.4 to 16.2 ms, 100-cell slab, which has no jumps, 1.37 to 1.25,
+        // Voronoi 2.71 to 2.57).
+        if constexpr (F::kJumpsLater) {
+            __syncwarp();
+            if (has && outcome == OUT_JUMP) {
+                int err = 0;
+                ++rws;
+                outcome = F::jump(C, t, rng, tal, err);
+                if (outcome == OUT_ERROR) {
+                    raise_error(C, err, F::cell(t), pid);
+                } else if (outcome == OUT_CONTINUE && segsThis >= maxSegs) {
+                    raise_error(C, STORM_DERR_HISTORY_CAP, F::cell(t), pid);
+                    outcome = OUT_ERROR;
                 }
             }
         }

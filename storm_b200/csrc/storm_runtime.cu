@@ -985,8 +985,12 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     h->fp32 = d->precision == STORM_PRECISION_FP32_TRACK;
     // measured on B200 at 64^3: FP32 tracking fits 64 registers without spills (4 blocks of 256
     // per SM); the FP64 form is fastest at 80 registers (3 blocks)
-    // FP64 on polyhedral meshes: 4 (Voronoi 1.2e4 cells, 1.8e7 segments: 2.64 against 2.80 ms with 3)
-    h->minBlocks = h->fp32 || d->mesh ? 4 : 3;
+    // Blocks a multiprocessor: 4 for FP32 and for the gray FP64 forms (64^3 cube 14.7
+    // against 16.2 ms with 3, Voronoi 2.64 against 2.80); 3 for the FP64 forms with the
+    // multigroup, DDMC or moving-material branches, which spill more (Densmore slab
+    // 9.9 against 10.8 ms with 4)
+    const bool gray64 = d->groups < 2 && !d->with_hydro && (d->mesh || !d->with_ddmc);
+    h->minBlocks = h->fp32 || gray64 ? 4 : 3;
     if (!poly) {
         std::vector<float> fx(d->nx), fy(d->ny), fz(d->nz);
         for (uint32_t i = 0; i < d->nx; ++i) fx[i] = static_cast<float>(0.5 * (h->hxe[i + 1] - h->hxe[i]));
