@@ -130,6 +130,8 @@ struct Ctx {
     unsigned long long *fixMat, *fixRad;
     double fixScaleMat, fixScaleRad;
     double *mgKTq;           // per cell: (kT)^q, written by the prestep
+    float4 *mg32;            // FP32-tracking form, per cell: kT, sigma0 / (kT)^q and the Random Walk's frequency
+                             // bound (rounded up), written when the transport begins (k_mg_cells)
     // DDMC-style leakage (RadiationIMCParameters::withDDMC)
     int32_t withDDMC;
     int32_t ddmcPgrw;        // ddmcUseMultigroupPGRW with a multigroup opacity
@@ -1501,8 +1503,8 @@ struct Track32 {
     // the cell's constants (enter_cell32), kept in registers while the particle stays in it
     float4 cp;
     float hx, hy, hz;
-    // multigroup: photon energy, and the cell's kT and sigma0 (cached with cp)
-    float nu, kT, s0;
+    // multigroup: photon energy, and the cell's kT, sigma0 / (kT)^q and PGRW frequency bound (with cp)
+    float nu, kT, s0, cut;
 };
 
 // the constants of the particle's cell, on a cell change along one axis without its half widths
@@ -1510,8 +1512,10 @@ template <bool MG>
 __device__ __forceinline__ void enter_cell32(const Ctx &C, Track32 &T) {
     T.cp = C.phys32[T.cell];
     if (MG) {
-        T.kT = static_cast<float>(mg_kT(C, T.cell));
-        T.s0 = static_cast<float>(C.sig0[T.cell] / C.mgKTq[T.cell]);   // sigma0 / (kT)^q
+        const float4 m = C.mg32[T.cell];
+        T.kT = m.x;
+        T.s0 = m.y;
+        T.cut = m.z;
     }
 }
 template <bool MG, bool POLY>
@@ -1932,7 +1936,7 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
     } else {
         Ro = nearest_face32<false>(C, T);
     }
-    if (Ro >= cp.z && Ro > 0.0f && (!MG || static_cast<double>(T.nu) < C.gb[C.pgrwCut[cell]])) {
+    if (Ro >= cp.z && Ro > 0.0f && (!MG || T.nu < T.cut)) {
         if constexpr (JUMPS) return OUT_JUMP;
         usedRW = 1;
         return rw_jump32<MG, POLY>(C, T, rng, tal, cp, Ro, hx, hy, hz, err);

@@ -143,6 +143,7 @@ void launch_transport_refill(cudaStream_t s, uint32_t grid, int minBlocks, const
 // chunkLevel: Q.chunks bytes; counts: 32 words; order: Q.chunks words
 void launch_chunk_order(cudaStream_t s, const uint32_t *cell, const uint8_t *level, uint32_t n, const RefillQueue &Q,
                         uint8_t *chunkLevel, uint32_t *counts, uint32_t *order);
+void launch_mg_cells(cudaStream_t s, const Ctx &C);   // before the transport, where C.mg32 is set
 void launch_fold_attenuation(cudaStream_t s, const Ctx &C, DevStats *st);   // after the transport, where C.att is set
 int refill_blocks_per_sm(int minBlocks, bool fp32);
 void launch_bank_to_local(cudaStream_t s, const Ctx &C, const Bank &src, const Bank &dst, uint32_t n,

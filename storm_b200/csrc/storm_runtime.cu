@@ -61,6 +61,7 @@ struct StormHandle {
     double *gb = nullptr;            // multigroup bounds
     float *gb32 = nullptr, *gc32 = nullptr;   // multigroup bounds and centres, FP32-tracking form
     double *faceCdf = nullptr;                // multigroup: 6 x (groups + 1) face Planck spectra
+    float4 *mg32 = nullptr;          // FP32 multigroup: per-cell constants of the transport (k_mg_cells)
     double *mgEp = nullptr, *mgKTq = nullptr; // multigroup: E_g^p per group, (kT)^q per cell
     double4 *ddmc = nullptr;                  // DDMC per-cell data, leak rates, FP32 copy
     double *ddmcTot = nullptr, *ddmcRate = nullptr;
@@ -1221,6 +1222,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
         ALLOC(A.pgrwCut, N);
         ALLOC(h->faceCdf, 6 * (static_cast<size_t>(G) + 1));
         ALLOC(h->mgKTq, N);
+        if (h->fp32) ALLOC(h->mg32, N);
         {
             // E^p at each group centre with the host's pow, as the opacity
             // model evaluates CalcAbsorptionOpacity there
@@ -1244,7 +1246,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
         C.sig0 = h->tabA;
         C.mgCdf = A.mgCdf; C.pgrw = A.pgrw; C.pgrwCut = A.pgrwCut;
         C.faceCdf = h->faceCdf;
-        C.mgEp = h->mgEp; C.mgEp32 = h->mgEp32; C.mgKTq = h->mgKTq;
+        C.mgEp = h->mgEp; C.mgEp32 = h->mgEp32; C.mgKTq = h->mgKTq; C.mg32 = h->mg32;
         if (h->fp32) {
             std::vector<float> b32(G + 1), c32(G);
             for (uint32_t g = 0; g <= G; ++g) b32[g] = static_cast<float>(d->group_bounds[g]);
@@ -1370,7 +1372,7 @@ int storm_cuda_destroy(StormHandle *h) {
                   h->A.rwElig, h->A.photons, h->A.phys, h->A.phys32, h->hx, h->hy, h->hz, h->segs, h->beginCounts, h->tabA, h->tabS, h->rhoF,
                   h->fsCell, h->fsSide, h->fsOffset, h->fsFace, h->fsArea, h->dAmbiguous, h->offsets, h->tileSums, h->dTotalU64, h->dTotalE, h->combW, h->combWtot,
                   h->combStart, h->combCount, h->combOff, h->counts, h->dStats, h->dErr, h->gb, h->A.mgCdf, h->A.pgrw,
-                  h->A.pgrwCut, h->gb32, h->gc32, h->faceCdf, h->mgEp, h->mgEp32, h->mgKTq, h->ddmc, h->ddmcTot,
+                  h->A.pgrwCut, h->gb32, h->gc32, h->faceCdf, h->mgEp, h->mgEp32, h->mgKTq, h->mg32, h->ddmc, h->ddmcTot,
                   h->ddmcRate, h->ddmcCut, h->ddmc32, h->stratBounds, h->stratBinW, h->stratStart,
                   h->runCursor, h->runScan, h->longRuns, h->bucketFlags,
                   h->cfo, h->cfN, h->cfP, h->cfNext, h->cfFace, h->mpx, h->mpy, h->mpz, h->fvo, h->fvi, h->vtx,
@@ -1644,6 +1646,10 @@ int storm_cuda_phase_transport(StormHandle *h) {
             if (h->profiling && h->evPool.empty()) {
                 h->evPool.resize(8);
                 for (auto &e : h->evPool) CK(cudaEventCreate(&e));
+            }
+            if (h->mg32) {
+                launch_mg_cells(h->stream, h->C);
+                ++h->launches;
             }
             RefillQueue Q = refill_queue(h, 0, n32);
             // Long histories first, where the bank is up to eight times what starts at
@@ -2290,6 +2296,10 @@ static int step_host_overlapped(StormHandle *h, double dt, const StormParticlesS
         const uint32_t need = static_cast<uint32_t>((len + 255) / 256);
         return need < g ? (need ? need : 1u) : g;
     };
+    if (h->mg32) {
+        launch_mg_cells(h->stream, h->C);
+        ++h->launches;
+    }
     if (nb > n) {
         launch_transport_refill(h->stream, grid_for_range(nb - n), h->minBlocks, h->C, h->bankA,
                                 refill_queue(h, n, nb), h->bankC, nCen,
