@@ -73,7 +73,7 @@ struct StormHandle {
     uint32_t *cfo = nullptr, *cfNext = nullptr, *cfFace = nullptr, *fvo = nullptr, *fvi = nullptr;
     double4 *cfN = nullptr, *cfP = nullptr;
     double *mpx = nullptr, *mpy = nullptr, *mpz = nullptr, *vtx = nullptr, *chord = nullptr;
-    float4 *cfN32 = nullptr;
+    float4 *cfN32 = nullptr, *cfX32 = nullptr;
     uint32_t *tetOff = nullptr;  // polyhedral emission: the cells' fan tetrahedra (k_poly_tets)
     double *tetCum = nullptr;
     uint2 *tetAT = nullptr;
@@ -1105,6 +1105,17 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
                 }
             ALLOC(h->cfN32, K);
             H2D(h->cfN32, pl.data(), K);
+            std::vector<float4> cross(K);
+            for (uint32_t c = 0; c < N; ++c)
+                for (uint32_t q = mesh->cell_face_offset[c]; q < mesh->cell_face_offset[c + 1]; ++q) {
+                    const uint32_t nb = nextv[q], at = nb < N ? nb : c;   // a ghost has no mesh point
+                    float bits;
+                    std::memcpy(&bits, &nb, sizeof(bits));
+                    cross[q] = make_float4(static_cast<float>(mp[0][c] - mp[0][at]), static_cast<float>(mp[1][c] - mp[1][at]),
+                                           static_cast<float>(mp[2][c] - mp[2][at]), bits);
+                }
+            ALLOC(h->cfX32, K);
+            H2D(h->cfX32, cross.data(), K);
         }
     }
     H2D(A.T, d->temperature, N);
@@ -1201,7 +1212,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
         C.poly = 1;
         C.cfo = h->cfo; C.cfN = h->cfN; C.cfP = h->cfP; C.cfNext = h->cfNext; C.cfFace = h->cfFace; C.cfA = h->cfA;
         C.mpx = h->mpx; C.mpy = h->mpy; C.mpz = h->mpz;
-        C.fvo = h->fvo; C.fvi = h->fvi; C.vtx = h->vtx; C.chord = h->chord; C.cfN32 = h->cfN32;
+        C.fvo = h->fvo; C.fvi = h->fvi; C.vtx = h->vtx; C.chord = h->chord; C.cfN32 = h->cfN32; C.cfX32 = h->cfX32;
         if (h->tetCum) {
             launch_poly_tets(h->stream, C, h->tetOff, h->tetCum, h->tetAT);
             if (cudaGetLastError() != cudaSuccess) return fail(STORM_ERR_CUDA);
@@ -1376,7 +1387,7 @@ int storm_cuda_destroy(StormHandle *h) {
                   h->ddmcRate, h->ddmcCut, h->ddmc32, h->stratBounds, h->stratBinW, h->stratStart,
                   h->runCursor, h->runScan, h->longRuns, h->bucketFlags,
                   h->cfo, h->cfN, h->cfP, h->cfNext, h->cfFace, h->mpx, h->mpy, h->mpz, h->fvo, h->fvi, h->vtx,
-                  h->chord, h->cfN32, h->dep, h->att, h->sumScratch, h->chunkCounts, h->A.level, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds, h->shardCount, h->shardOff, h->shardTiles,
+                  h->chord, h->cfN32, h->cfX32, h->dep, h->att, h->sumScratch, h->chunkCounts, h->A.level, h->xbuf, h->shardWc, h->shardRunW, h->shardStart, h->shardBounds, h->shardCount, h->shardOff, h->shardTiles,
                   h->vel, h->mom, h->ddmcCum32, h->cfA, h->egAvg, h->fixMat, h->fixRad, h->tetOff, h->tetCum,
                   h->tetAT};
     for (void *p : ps) device_pool().free(p);
