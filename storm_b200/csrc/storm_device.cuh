@@ -583,7 +583,7 @@ struct SegmentTallyFixed : SegmentTally {
 // planck_integral(a, b) = 15/pi^4 int_a^b x^3/(e^x - 1) dx from Clark's two
 // published series: the Bernoulli expansion below x = 0.5 and the exponential
 // tail series sum_n e^{-n x} (x^3/n + 3x^2/n^2 + 6x/n^3 + 6/n^4) above, with the
-// host table build's switch point and stopping rule.  On the device the tail's
+// host table build's switch point, taken until a term can't change the sum.  On the device the tail's
 // exponentials come by recurrence, e^{-(n+1)x} = e^{-nx} e^{-x}, and each term
 // takes one division; both change the sum by about n ulps (n < 100 terms
 // where x >= 0.5), far inside the 1e-12 the tables are held to.
@@ -591,7 +591,7 @@ constexpr double PI_NORM_PI = 3.14159265358979323846;
 __device__ __forceinline__ double pi_norm() { return 15.0 / (PI_NORM_PI * PI_NORM_PI * PI_NORM_PI * PI_NORM_PI); }
 // The series' constants, folded at compile time so that the device multiplies
 // instead of dividing: the small-x coefficients B_k / (k! (k + 3)), and 1/n^j
-// (j = 1..4) for the first PI_TAIL_TABLE tail terms.  Both change the sums by
+// (j = 1..3) and 6/n^4 for the tail terms.  Both change the sums by
 // a few ulps, inside the tables' 1e-12.
 struct PiSmallCoef {
     double c[21];
@@ -608,14 +608,14 @@ struct PiSmallCoef {
 };
 constexpr int PI_TAIL_TABLE = 128;
 struct PiTailInv {
-    double v[4 * PI_TAIL_TABLE];   // per n: 1/n, 1/n^2, 1/n^3, 1/n^4
+    double v[4 * PI_TAIL_TABLE];   // per n: 1/n, 1/n^2, 1/n^3, 6/n^4
     constexpr PiTailInv() : v() {
         for (int n = 1; n <= PI_TAIL_TABLE; ++n) {
             const double d = n, d2 = d * d;
             v[4 * (n - 1)] = 1.0 / d;
             v[4 * (n - 1) + 1] = 1.0 / d2;
             v[4 * (n - 1) + 2] = 1.0 / (d2 * d);
-            v[4 * (n - 1) + 3] = 1.0 / (d2 * d2);
+            v[4 * (n - 1) + 3] = 6.0 * (1.0 / (d2 * d2));
         }
     }
 };
@@ -623,40 +623,36 @@ static __constant__ PiSmallCoef c_piSmall = PiSmallCoef();
 static __constant__ PiTailInv c_piTail = PiTailInv();
 
 __device__ inline double pi_small_series(double x) {
-    // x^3 sum_k c_k x^k, the zero coefficients skipped, by Horner in x
+    // x^3 sum_k c_k x^k by Horner in x; B_k is zero for odd k > 1
     double sum = c_piSmall.c[20];
 #pragma unroll
-    for (int k = 19; k >= 0; --k) sum = sum * x + c_piSmall.c[k];
+    for (int k = 19; k >= 0; --k) {
+        sum = sum * x;
+        if (!(k & 1) || k == 1) sum = sum + c_piSmall.c[k];
+    }
     return sum * (x * x * x);
 }
-__device__ inline double pi_tail_series(double x) {
+__device__ inline double pi_tail_series(double x, const double *inv) {
     const double e1 = exp(-x);
     const double x2 = x * x, x3 = x2 * x;
     const double a2 = 3.0 * x2, a3 = 6.0 * x;
     double sum = 0.0, e = e1;
     const double e1sq = e1 * e1;
-    // every lane of a warp takes term n at the same time, so the table read is
-    // uniform; terms go in pairs, whose exponentials are two independent
-    // products, and the sum adds them in order
-    int n = 1;
-    for (; n + 1 <= PI_TAIL_TABLE && e != 0.0; n += 2) {
-        const double *iv = c_piTail.v + 4 * (n - 1);
+    // Every lane of a warp takes term n at the same time, so the table read (inv:
+    // c_piTail or a copy) is uniform; terms go in pairs, whose exponentials are two independent
+    // products, and the sum adds them in order.  The FP64 pipe bounds this loop,
+    // so the end is found on the words of the numbers, once a pair: a term under
+    // 2^-54 of the sum is under half its last place and the later ones are
+    // smaller still.  At x = 0.5, the smallest here, that is term 60.
+    for (int n = 1; n < PI_TAIL_TABLE && e != 0.0; n += 2) {
+        const double *iv = inv + 4 * (n - 1);
         const double eb = e * e1;
-        const double ta = e * (((x3 * iv[0] + a2 * iv[1]) + a3 * iv[2]) + 6.0 * iv[3]);
-        const double tb = eb * (((x3 * iv[4] + a2 * iv[5]) + a3 * iv[6]) + 6.0 * iv[7]);
+        const double ta = e * (((x3 * iv[0] + a2 * iv[1]) + a3 * iv[2]) + iv[3]);
+        const double tb = eb * (((x3 * iv[4] + a2 * iv[5]) + a3 * iv[6]) + iv[7]);
         sum += ta;
-        if (ta < 1e-18 * sum) return sum;
         sum += tb;
-        if (tb < 1e-18 * sum) return sum;
+        if (__double2hiint(tb) + (54 << 20) < __double2hiint(sum)) break;
         e *= e1sq;
-    }
-    for (; n < 100000 && e != 0.0; ++n) {
-        const double dn = n;
-        const double d2 = dn * dn;
-        const double term = e * ((((x3 * dn + a2) * dn + a3) * dn + 6.0) / (d2 * d2));
-        sum += term;
-        if (term < 1e-18 * sum) break;
-        e *= e1;
     }
     return sum;
 }
@@ -666,13 +662,13 @@ __device__ inline double pi_tail_series(double x) {
 struct PiBound {
     double x, tail, cum;
 };
-__device__ inline PiBound pi_bound(double x) {
+__device__ inline PiBound pi_bound(double x, const double *inv = c_piTail.v) {
     PiBound r{x, 0.0, 0.0};
     if (!(x > 0.0)) return r;
     if (x < 0.5) {
         r.cum = pi_norm() * pi_small_series(x);
     } else {
-        r.tail = pi_tail_series(x);
+        r.tail = pi_tail_series(x, inv);
         r.cum = 1.0 - pi_norm() * r.tail;
     }
     return r;

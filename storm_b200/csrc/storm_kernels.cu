@@ -330,7 +330,8 @@ __device__ __forceinline__ void cell_rw_and_phys32(const Ctx &C, const CellArray
 // spectrum sum_g sigma_g B_g it samples from (:146-165), and the PGRW data of
 // precomputeRandomWalkData (radiation/RadiationIMC.hpp:1008-1061).  Every
 // group weight is evaluated at the group centre with planck_integral.
-__device__ inline double mg_cell_tables(const Ctx &C, const CellArrays &A, uint32_t c, double scat, double chord) {
+__device__ inline double mg_cell_tables(const Ctx &C, const CellArrays &A, uint32_t c, double scat, double chord,
+                                        const double *tailInv) {
     const uint32_t G = C.groups;
     const double T = C.T[c];
     const double kT = C.kBoltz * (T < 1.0 ? 1.0 : T);   // the opacity model's kT
@@ -343,11 +344,11 @@ __device__ inline double mg_cell_tables(const Ctx &C, const CellArrays &A, uint3
     cdf[0] = 0.0;
     const double kTq = pow(kT, C.mgQ);   // the same in every group
     C.mgKTq[c] = kTq;
-    PiBound lo = pi_bound(C.gb[0] / kT);
+    PiBound lo = pi_bound(C.gb[0] / kT, tailInv);
     for (uint32_t g = 0; g < G; ++g) {
         const double b0 = C.gb[g], b1 = C.gb[g + 1];
         const double Ec = 0.5 * (b0 + b1);
-        const PiBound hi = pi_bound(b1 / kT);
+        const PiBound hi = pi_bound(b1 / kT, tailInv);
         const double a = lo.x, b = hi.x;   // b0 / kT, b1 / kT
         const double Bg = (a > 0.0 && b > a) ? pi_between(lo, hi) : 0.0;
         lo = hi;
@@ -456,13 +457,27 @@ __device__ __forceinline__ uint8_t history_level(double sa, double ss, double f,
     const int l = events > 1.0 ? ilogb(events) : 0;
     return static_cast<uint8_t>(l > 15 ? 15 : l);
 }
-__global__ void k_prestep(Ctx C, CellArrays A, OpacityEos M, double dt) {
+// The multigroup form is bound by the FP64 pipe and its latencies (G + 1 Planck
+// series and G expm1 a cell); it reads the series' constants from shared memory,
+// since indexed constant loads held their own pipe at 57 % of its rate.  72^3 x 64
+// groups: 867 us when every term was tested in FP64, 722 us with the end of a
+// series found on the words, 678 us in blocks of 128 with the table in shared
+// memory; six or eight blocks a multiprocessor instead of four spill and take the
+// emission phase of 40^3 cells from 0.375 to 0.39 and 0.41 ms.
+constexpr int PRESTEP_THREADS = 128;
+template <bool MG>
+__global__ void __launch_bounds__(PRESTEP_THREADS, MG ? 4 : 1) k_prestep(Ctx C, CellArrays A, OpacityEos M, double dt) {
+    __shared__ double tailInv[MG ? 4 * PI_TAIL_TABLE : 1];
+    if constexpr (MG) {
+        for (int q = threadIdx.x; q < 4 * PI_TAIL_TABLE; q += PRESTEP_THREADS) tailInv[q] = c_piTail.v[q];
+        __syncthreads();
+    }
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < C.ncells; c += gridDim.x * blockDim.x) {
         double sa, ss;
         const double T = A.T[c];
-        if (C.groups >= 2) {
+        if constexpr (MG) {
             ss = M.tabS ? M.tabS[c] : 0.0;
-            sa = mg_cell_tables(C, A, c, ss, C.withRW ? cell_chord(C, A, c) : 0.0);
+            sa = mg_cell_tables(C, A, c, ss, C.withRW ? cell_chord(C, A, c) : 0.0, tailInv);
         } else if (M.opacityKind == STORM_OPACITY_CELL_TABLE) {
             sa = M.tabA[c];
             ss = M.tabS ? M.tabS[c] : 0.0;
@@ -3557,7 +3572,9 @@ void launch_begin(cudaStream_t s, const Bank &b, uint32_t n, uint32_t pidOffset,
     if (n > lo) k_begin<<<grid_for(n - lo, 256, 4096), 256, 0, s>>>(b, lo, n, pidOffset, dt, st);
 }
 void launch_prestep(cudaStream_t s, const Ctx &C, const CellArrays &A, const OpacityEos &M, double dt) {
-    k_prestep<<<grid_for(C.ncells, 256, 8192), 256, 0, s>>>(C, A, M, dt);
+    const uint32_t grid = grid_for(C.ncells, PRESTEP_THREADS, 16384);
+    if (C.groups >= 2) k_prestep<true><<<grid, PRESTEP_THREADS, 0, s>>>(C, A, M, dt);
+    else k_prestep<false><<<grid, PRESTEP_THREADS, 0, s>>>(C, A, M, dt);
 }
 void launch_ddmc_rates(cudaStream_t s, const Ctx &C, const CellArrays &A) {
     k_ddmc_rates<<<grid_for(C.ncells, 256, 8192), 256, 0, s>>>(C, A);

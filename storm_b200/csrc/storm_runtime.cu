@@ -145,7 +145,7 @@ struct StormHandle {
     uint64_t *shardBounds = nullptr; // 3 (S + 1) pid bounds (Ctx::shardBounds)
     uint32_t step = 0;
     uint32_t K = 8, maxRounds = 4096;
-    int minBlocks = 3;               // transport occupancy variant (__launch_bounds__ min blocks); 4 for FP32
+    int minBlocks = 3;               // transport occupancy variant (__launch_bounds__ min blocks); 4 for FP32 and gray FP64
     int refill = 1;                  // 1: persistent refill kernel, 0: bank visits of K segments
     uint32_t burst = 8;              // refill kernel: segments between refills
     // online burst tuning (storm_cuda_autotune_transport): step k of the
@@ -984,9 +984,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     H2D(h->xe, h->hxe.data(), ex + 1); H2D(h->ye, h->hye.data(), ey + 1); H2D(h->ze, h->hze.data(), ez + 1);
     H2D(h->xc, h->hxc.data(), ex); H2D(h->yc, h->hyc.data(), ey); H2D(h->zc, h->hzc.data(), ez);
     h->fp32 = d->precision == STORM_PRECISION_FP32_TRACK;
-    // measured on B200 at 64^3: FP32 tracking fits 64 registers without spills (4 blocks of 256
-    // per SM); the FP64 form is fastest at 80 registers (3 blocks)
-    // Blocks a multiprocessor: 4 for FP32 and for the gray FP64 forms (64^3 cube 14.7
+    // Blocks a multiprocessor: 4 for FP32 (64 registers hold it) and for the gray FP64 forms (64^3 cube 14.7
     // against 16.2 ms with 3, Voronoi 2.64 against 2.80); 3 for the FP64 forms with the
     // multigroup, DDMC or moving-material branches, which spill more (Densmore slab
     // 9.9 against 10.8 ms with 4)
