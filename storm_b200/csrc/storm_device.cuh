@@ -26,7 +26,7 @@ enum : int { JUMP = 7 };   // a Random Walk jump that the caller takes later (ju
 enum : int { OUT_CONTINUE = 0, OUT_CENSUS = 1, OUT_CUTOFF = 2, OUT_ESCAPE = 3, OUT_ERROR = -1 };
 // left by a segment of the persistent transport for its finish (finish64, finish32)
 enum : int { OUT_SCATTER = 4, OUT_REEMIT = 5 };
-enum : int { OUT_JUMP = 6 };   // a Random Walk jump for the end of the burst (jump64, jump32)
+enum : int { OUT_JUMP = 6 };   // a Random Walk jump for the end of the burst (jump64)
 // random stream tags
 enum : uint32_t { TAG_TRANSPORT = 1, TAG_CELL_EMIT = 2, TAG_FACE_EMIT = 3, TAG_COMB = 4 };
 
@@ -1905,14 +1905,7 @@ __device__ __forceinline__ float nearest_face32(const Ctx &C, const Track32 &T) 
         return fminf(fminf(T.hx - fabsf(T.qx), T.hy - fabsf(T.qy)), T.hz - fabsf(T.qz));
     }
 }
-// The Random Walk jump that a segment left (OUT_JUMP), gray
-template <bool POLY, class RNG, class TALLY>
-__device__ inline int jump32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, int &err) {
-    return rw_jump32<false, POLY>(C, T, rng, tal, T.cp, nearest_face32<POLY>(C, T), T.hx, T.hy, T.hz, err);
-}
-
-// JUMPS leaves a Random Walk jump (OUT_JUMP) to jump32.
-template <bool MG, bool LATER, bool JUMPS, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
+template <bool MG, bool LATER, class RNG, class TALLY, bool POLY = false, bool DDMC = true>
 __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, int &usedRW, int &err) {
     const uint32_t cell = T.cell;
     // the draws a segment can take: the collision and the scatter's two; in a
@@ -1937,7 +1930,6 @@ __device__ inline int segment32(const Ctx &C, Track32 &T, RNG &rng, TALLY &tal, 
         Ro = nearest_face32<false>(C, T);
     }
     if (Ro >= cp.z && Ro > 0.0f && (!MG || T.nu < T.cut)) {
-        if constexpr (JUMPS) return OUT_JUMP;
         usedRW = 1;
         return rw_jump32<MG, POLY>(C, T, rng, tal, cp, Ro, hx, hy, hz, err);
     }

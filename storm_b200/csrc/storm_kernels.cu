@@ -1502,7 +1502,7 @@ using Form64PolyDDMCFix = Form64T<5, SegmentTallyFixed>;
 template <bool POLY, bool DDMC = true, class TL = SegmentTally>
 struct Form32T {
     static constexpr bool kTogether = POLY;
-    static constexpr bool kJumpsLater = false;   // 64^3 5.7 to 5.8 ms, 24^3 0.47 to 0.49, served problems 75 to 72
+    static constexpr bool kJumpsLater = false;   // later, 64^3 took 5.8 for 5.7 ms, 24^3 0.49 for 0.47
     using T = Track32;
     using Rng = PhiloxRng4;      // bank visits
     using Ring = PhiloxRing4;    // the persistent transport
@@ -1520,17 +1520,13 @@ struct Form32T {
     }
     template <bool LATER, bool JUMPS, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<false, LATER, JUMPS, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<false, LATER, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
         return m;
     }
     template <class RNG>
     static __device__ __forceinline__ bool finish(const Ctx &C, T &t, RNG &rng, int) {
         return finish32<false>(C, t, rng, true);
-    }
-    template <class RNG, class TALLY>
-    static __device__ __forceinline__ int jump(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &err) {
-        return jump32<POLY>(C, t, rng, tal, err);
     }
     static __device__ __forceinline__ uint32_t cell(const T &t) { return t.cell; }
     static __device__ __forceinline__ double weight(const T &t) { return t.w; }
@@ -1567,7 +1563,7 @@ struct Form32MGT {
     }
     template <bool LATER, bool JUMPS, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
-        int m = segment32<true, LATER, false, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
+        int m = segment32<true, LATER, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
         if (m == OUT_CONTINUE && t.nu < 0.0f) m = OUT_REEMIT;   // a Random Walk's upscatter
         return m;
