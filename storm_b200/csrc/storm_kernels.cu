@@ -5,6 +5,7 @@
 
 #include <type_traits>
 
+#include "storm_comb.cuh"
 #include "storm_device.cuh"
 #include "storm_internal.h"
 
@@ -2686,16 +2687,6 @@ __device__ __forceinline__ uint64_t teeth_below(double P, double r, double E) {
     return k;
 }
 
-// teeth_below for P > 0 from a guess P * perE (perE about 1 / E), with the index
-// as a whole number in FP64: the index follows from the comparisons, not from the
-// guess, and costs neither a division nor 64-bit integer conversions.
-__device__ __forceinline__ double teeth_index(double P, double perE, double r, double E) {
-    double k = fmax(ceil(P * perE - r), 0.0);
-    while (k > 0.0 && ((k - 1.0) + r) * E >= P) k -= 1.0;
-    while ((k + r) * E < P) k += 1.0;
-    return k;
-}
-
 // s with x added n times, one after another (s >= 0, x > 0).  While the sum stays
 // in one binade each addition moves it by the same multiple d of the binade's
 // unit u, unless x lies halfway between two multiples; so a whole binade is one
@@ -2831,14 +2822,14 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
                 m = made;
             }
         } else {   // comb
-            const double r = __shfl_sync(FULL, cc.r, l), newEnergy = __shfl_sync(FULL, cc.e, l);
-            const double perE = 1.0 / newEnergy;
+            const double newEnergy = __shfl_sync(FULL, cc.e, l);
+            const CombTeeth teeth = comb_teeth(__shfl_sync(FULL, cc.r, l), newEnergy, __shfl_sync(FULL, cc.nin, l));
             double before = 0.0;   // the comb index at the particle before
             double p = ra + lane < rb ? upTo[ra + lane] : 0.0;
             for (uint32_t base = ra; base < rb; base += 32) {
                 const uint32_t q = base + lane;
                 const bool in = q < rb;
-                const double k = in ? teeth_index(p, perE, r, newEnergy) : 0.0;
+                const double k = in ? teeth_index(teeth, p) : 0.0;
                 p = q + 32 < rb ? upTo[q + 32] : 0.0;
                 double k0 = __shfl_up_sync(FULL, k, 1);
                 if (lane == 0) k0 = before;
