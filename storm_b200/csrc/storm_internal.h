@@ -128,7 +128,7 @@ void launch_strat_sums(cudaStream_t s, const double *wS, const uint32_t *start, 
 void launch_strat_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const StratParams &S, const double *wS,
                        const uint32_t *start, const double *binW, const double *cellW, const double *Wtot,
                        uint32_t *pCount, double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
-                       DevStats *st);
+                       DevStats *st, const uint32_t *unsorted);
 void launch_face_spectra(cudaStream_t s, const Ctx &C, double *cdf);
 void launch_set_u32(cudaStream_t s, uint32_t *p, uint32_t v);
 void launch_poly_tets(cudaStream_t s, const Ctx &C, const uint32_t *tetOff, double *tetCum, uint2 *tetAT);
@@ -168,9 +168,10 @@ void launch_comb_cell_sums(cudaStream_t s, const double *wS, const uint32_t *sta
                            double *W, double *upTo = nullptr);
 // scratch: 1025 doubles, the last zero (NULL: one block sums)
 void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out, double *scratch = nullptr);
+// unsorted: where it is not NULL and set, the plan does nothing
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
-                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st);
+                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st, const uint32_t *unsorted);
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,
                       const uint32_t *pOff, const uint64_t *groupOff, const Bank &out);

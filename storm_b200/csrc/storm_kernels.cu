@@ -2723,13 +2723,16 @@ __device__ __noinline__ double add_repeated(double s, double x, uint64_t n) {
 // that is kept or split the energy is the running weight, too, up to the first
 // particle that is split; only from there on is there a serial chain, over the
 // copies, which are laid out in shared memory for it.  pOff: a particle's first
-// copy among its cell's.
+// copy among its cell's.  unsorted: set where the bucket sort met a run too long for
+// it, whose sorted weights nobody has written; the plan then leaves everything as it
+// is, for the one that follows the radix sort.
 __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams P, const double *wS,
                                                                const uint32_t *start, const double *W,
                                                                const double *upTo, const double *Wtot,
                                                                uint32_t *pCount, double *pWeight, uint32_t *pOff,
                                                                uint64_t *cellCount, double *eradCensus, DevStats *st,
-                                                               uint32_t batch) {
+                                                               const uint32_t *unsorted, uint32_t batch) {
+    if (unsorted && *unsorted) return;
     constexpr uint32_t COPIES = 256;   // copies of 32 particles that are laid out for the chain
     __shared__ __align__(16) double stage[WALK_WARPS][COPIES + 8];
     const double tot = *Wtot;
@@ -2855,7 +2858,8 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
 // The same plan with a thread per cell (walk_by_thread).
 __global__ void k_comb_plan_thread(Ctx C, CombParams P, const double *wS, const uint32_t *start, const double *W,
                                    const double *Wtot, uint32_t *pCount, double *pWeight, uint32_t *pOff,
-                                   uint64_t *cellCount, double *eradCensus, DevStats *st) {
+                                   uint64_t *cellCount, double *eradCensus, DevStats *st, const uint32_t *unsorted) {
+    if (unsorted && *unsorted) return;
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -3271,7 +3275,8 @@ __global__ void k_strat_sums(const double *wS, const uint32_t *start, uint32_t n
 __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *wS, const uint32_t *start,
                              const double *binW, const double *cellW, const double *Wtot, uint32_t *pCount,
                              double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
-                             DevStats *st) {
+                             DevStats *st, const uint32_t *unsorted) {
+    if (unsorted && *unsorted) return;
     const double tot = *Wtot;
     if (!isfinite(tot)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
@@ -3667,9 +3672,9 @@ void launch_strat_sums(cudaStream_t s, const double *wS, const uint32_t *start, 
 void launch_strat_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const StratParams &S, const double *wS,
                        const uint32_t *start, const double *binW, const double *cellW, const double *Wtot,
                        uint32_t *pCount, double *pWeight, uint32_t *pOff, uint64_t *cellCount, double *eradCensus,
-                       DevStats *st) {
+                       DevStats *st, const uint32_t *unsorted) {
     k_strat_plan<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, S, wS, start, binW, cellW, Wtot, pCount, pWeight,
-                                                             pOff, cellCount, eradCensus, st);
+                                                             pOff, cellCount, eradCensus, st, unsorted);
 }
 void launch_transport(cudaStream_t s, uint32_t grid, const Ctx &C, const Bank &in, const uint32_t *nIn, const Bank &out,
                       uint32_t *nOut, const CensusBank &cen, uint32_t *nCen, uint32_t K, DevStats *st, int minBlocks) {
@@ -3800,14 +3805,14 @@ void launch_blocked_sum(cudaStream_t s, const double *v, uint32_t n, double *out
 }
 void launch_comb_plan(cudaStream_t s, const Ctx &C, const CombParams &P, const double *wS, const uint32_t *start,
                       uint32_t n, const double *W, const double *upTo, const double *Wtot, uint32_t *pCount, double *pWeight,
-                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st) {
+                      uint32_t *pOff, uint64_t *cellCount, double *eradCensus, DevStats *st, const uint32_t *unsorted) {
     if (walk_by_thread(n, C.ncells)) {
         k_comb_plan_thread<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, P, wS, start, W, Wtot, pCount, pWeight,
-                                                                         pOff, cellCount, eradCensus, st);
+                                                                         pOff, cellCount, eradCensus, st, unsorted);
         return;
     }
     k_comb_plan<<<walk_grid(C.ncells), 32 * WALK_WARPS, 0, s>>>(C, P, wS, start, W, upTo, Wtot, pCount, pWeight,
-                                                                pOff, cellCount, eradCensus, st, walk_batch(C.ncells));
+                                                                pOff, cellCount, eradCensus, st, unsorted, walk_batch(C.ncells));
 }
 void launch_comb_emit(cudaStream_t s, const Ctx &C, const CensusBank &cen, const uint32_t *idx, const uint64_t *sortedKeys,
                       int pidBits, uint32_t bins, uint32_t nValid, const uint32_t *pCount, const double *pWeight,

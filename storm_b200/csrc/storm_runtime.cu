@@ -1986,18 +1986,19 @@ int storm_cuda_phase_comb(StormHandle *h) {
         launch_sorted_weights(h->stream, h->C, h->bankC, idx, n, wS);
         h->launches += 5 * ((pidBits + cellBits + 7) / 8) + 2;
     };
-    // per-cell sums, the plan, and the scan of the cells' copies
-    auto plan_and_scan = [&]() {
+    // per-cell sums, the plan, and the scan of the cells' copies (of no meaning where
+    // the bucket sort failed: its flag, which the plan reads)
+    auto plan_and_scan = [&](const uint32_t *unsorted) {
         pOff = reinterpret_cast<uint32_t *>(skeys == h->keysAlt ? h->keys : h->keysAlt);
         if (strat) launch_strat_sums(h->stream, wS, start, N, B, h->stratBinW, h->combW);
         else launch_comb_cell_sums(h->stream, wS, start, n, N, h->combW, upTo);
         launch_blocked_sum(h->stream, h->combW, N, h->combWtot, h->sumScratch);
         if (strat)
             launch_strat_plan(h->stream, h->C, P, h->strat, wS, start, h->stratBinW, h->combW, h->combWtot, h->pCount,
-                              h->pWeight, pOff, h->combCount, h->A.eradCensus, h->dStats);
+                              h->pWeight, pOff, h->combCount, h->A.eradCensus, h->dStats, unsorted);
         else
             launch_comb_plan(h->stream, h->C, P, wS, start, n, h->combW, upTo, h->combWtot, h->pCount, h->pWeight,
-                             pOff, h->combCount, h->A.eradCensus, h->dStats);
+                             pOff, h->combCount, h->A.eradCensus, h->dStats, unsorted);
         launch_scan_u64(h->stream, h->combCount, N, h->combOff, h->tileSums, h->dTotalU64);
         h->launches += 3 + scan_launches(N);
     };
@@ -2028,7 +2029,7 @@ int storm_cuda_phase_comb(StormHandle *h) {
     } else {
         radix_sort();
     }
-    plan_and_scan();
+    plan_and_scan(bucket ? h->bucketFlags + 1 : nullptr);
     CK(cudaGetLastError());
     uint32_t flags[2] = {0, 0};
     uint32_t nValid = 0;
@@ -2040,15 +2041,10 @@ int storm_cuda_phase_comb(StormHandle *h) {
         if (rc != STORM_OK) return rc;
     }
     if (bucket && flags[1]) {
-        // a run too long for the bucket sort: sort by radix and plan again (the
-        // plan adds the census energy to the step statistics, so that restarts)
-        CK(cudaMemsetAsync(&h->dStats->eCensusOut, 0, sizeof(double), h->stream));
-        // the keys again: the first plan's copy offsets went to their buffer
-        if (strat) launch_strat_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits, h->strat);
-        else launch_comb_keys(h->stream, h->C, h->bankC, n, h->keys, h->vals, combKey, pidBits);
-        ++h->launches;
+        // a run too long for the bucket sort: sort by radix, then plan (the first plan
+        // left everything as it was, the keys too)
         radix_sort();
-        plan_and_scan();
+        plan_and_scan(nullptr);
         CK(cudaGetLastError());
         const Readback r[2] = {{&nValid, start + nRuns, sizeof(uint32_t)}, {&total, h->dTotalU64, sizeof(uint64_t)}};
         const int rc = read_many(h, r, 2, true);

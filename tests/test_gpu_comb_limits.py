@@ -1,8 +1,9 @@
 """The comb at the ends of what it accepts: census weights down to the smallest
-doubles."""
+doubles, and cells of more particles than a block sorts."""
 import numpy as np
 import pytest
 
+from storm_b200 import _abi as A
 from storm_b200 import problems
 from storm_b200.engine import Engine
 
@@ -51,3 +52,36 @@ def test_smallest_weights(oracle_lib, unit, nx):
     cell = np.repeat(rng.permutation(nx)[:4 * len(lengths)], np.tile(lengths, 4))
     weight = np.ceil(1000.0 * rng.random(len(cell))) * unit
     same_as_oracle(oracle_lib, p, Engine(p), census(p, cell, weight))
+
+
+@pytest.mark.parametrize("longest", [8192, 8193, 20000])
+@pytest.mark.parametrize("kind", ["plain", "stratified"])
+def test_long_runs_on_a_used_block(oracle_lib, kind, longest):
+    """A cell whose run is sorted by radix after the first plan has been launched: that
+    plan must not touch the weights the first sort left unwritten, here those of
+    another handle's last comb on the same memory."""
+    def problem():
+        p = problems.gray_slab(nx=6, new_photons_per_cell=1, face_packets=10, comb_nmin=2000, comb_factor=1.5)
+        if kind == "stratified":
+            p.comb_kind = A.COMB_STRATIFIED
+        return p
+    p = problem()
+    n = 6 * 7000
+    first = Engine(p)   # tiny weights in every slot of the buffers
+    first.population_control(census(p, np.repeat(np.arange(6), 7000), np.full(n, 1e-309)))
+    first.close()
+    e = Engine(problem())
+    cell = np.concatenate([np.full(longest, 2), np.array([0, 1, 3, 4, 5])[np.arange(n - longest) % 5]]).astype(np.uint32)
+    weight = np.exp(np.random.default_rng(longest).standard_normal(n))
+    pre = census(p, cell, weight)
+    if kind == "plain":
+        same_as_oracle(oracle_lib, problem(), e, pre)
+        return
+    a = e.population_control(pre)
+    energy = e.cells()["erad_census"]
+    b = e.population_control(pre)
+    assert a.n == b.n > 0
+    np.testing.assert_array_equal(a.cell, b.cell)
+    np.testing.assert_array_equal(a.weight, b.weight)
+    np.testing.assert_array_equal(energy, e.cells()["erad_census"])
+    np.testing.assert_allclose(a.weight.sum(), weight.sum(), rtol=1e-9)
