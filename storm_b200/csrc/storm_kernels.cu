@@ -2660,6 +2660,13 @@ struct CombCell {
     int mode;         // 0 keep/split, 1 comb
 };
 
+// The weight that kept or split particles aim at, total / n.  Where it is below the
+// smallest double, so is a share of any particle: infinity, which splits none.
+__device__ __forceinline__ double split_weight(double total, double n) {
+    const double w = total / n;
+    return w > 0.0 ? w : CUDART_INF;
+}
+
 __device__ __forceinline__ CombCell comb_cell_params(const Ctx &C, const CombParams &P, uint32_t c, uint32_t cnt,
                                                      double Wc, double Wtot) {
     CombCell cc;
@@ -2667,7 +2674,7 @@ __device__ __forceinline__ CombCell comb_cell_params(const Ctx &C, const CombPar
     uint64_t lo = share > P.nmin ? share : P.nmin;
     cc.nin = (P.nmin * 20 < lo) ? P.nmin * 20 : lo;
     cc.mode = (cnt <= cc.nin) ? 0 : 1;
-    cc.w_ideal = Wc / static_cast<double>(cc.nin);
+    cc.w_ideal = split_weight(Wc, static_cast<double>(cc.nin));
     cc.e = cc.w_ideal;
     cc.r = cc.mode ? stream_uniform(C.seedLo, C.seedHi, TAG_COMB, C.step, c, 0) : 0.0;
     return cc;
@@ -3349,7 +3356,7 @@ __global__ void k_strat_plan(Ctx C, CombParams P, StratParams S, const double *w
                 if (tg == 0 || !(bw > 0.0)) {   // a bin without a target loses its particles (:349-350)
                     for (uint32_t q = a; q < b; ++q) pCount[q] = 0;
                 } else if (static_cast<uint64_t>(b - a) <= tg) {
-                    const double ideal = bw / static_cast<double>(tg);
+                    const double ideal = split_weight(bw, static_cast<double>(tg));
                     for (uint32_t q = a; q < b; ++q) {
                         const double w = wS[q];
                         if (w > 2.0 * ideal) {

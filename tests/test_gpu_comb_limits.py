@@ -85,3 +85,23 @@ def test_long_runs_on_a_used_block(oracle_lib, kind, longest):
     np.testing.assert_array_equal(a.weight, b.weight)
     np.testing.assert_array_equal(energy, e.cells()["erad_census"])
     np.testing.assert_allclose(a.weight.sum(), weight.sum(), rtol=1e-9)
+
+
+@pytest.mark.parametrize("nx", [20, 100003])   # by warps, and a thread per cell
+@pytest.mark.parametrize("kind", ["plain", "stratified"])
+def test_weights_too_small_to_split_are_kept(kind, nx):
+    """A cell's share of the smallest double is zero: its particles stay as they are,
+    beside a cell of ordinary ones that are split."""
+    p = problems.gray_slab(nx=nx, new_photons_per_cell=1, face_packets=10, comb_nmin=50, comb_factor=1.5)
+    if kind == "stratified":
+        p.comb_kind = A.COMB_STRATIFIED
+    tiny = 4.94065645841246544e-324
+    pre = census(p, np.array([3, 7, 7, 11, 11, 11]), [tiny, tiny, 2 * tiny, 1.0, 0.5, 0.25])
+    e = Engine(p)
+    for _ in range(2):   # the second time the banks hold the split particles
+        post = e.population_control(pre)
+        np.testing.assert_array_equal(post.weight[post.cell == 3], [tiny])
+        np.testing.assert_array_equal(np.sort(post.weight[post.cell == 7]), [tiny, 2 * tiny])
+        hot = post.weight[post.cell == 11]
+        assert len(hot) >= 50 and abs(hot.sum() - 1.75) < 1e-12 and (hot > 0).all()
+        assert post.n == 3 + len(hot)
