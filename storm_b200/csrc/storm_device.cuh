@@ -1475,7 +1475,7 @@ __device__ inline PhysOut physics_step(const Ctx &C, Track &T, RNG &rng, TALLY &
             return o;
         }
         const double oldVx = p.vx, oldVy = p.vy, oldVz = p.vz;
-        if (HYDRO) p.nu *= dop;   // dop = 1 for a cell at rest
+        if (HYDRO && C.groups >= 2) p.nu *= dop;   // dop = 1 for a cell at rest; gray: only lorentz_to_lab shifts it
         if (!finish64<FULL>(C, T, rng, effective)) { o.errCode = STORM_DERR_MG_SAMPLE; return o; }
         if (HYDRO && C.withHydro) {   // the comoving scatter back to the lab frame (:1853-1871)
             const double weightBefore = p.w;
