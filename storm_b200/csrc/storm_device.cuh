@@ -105,7 +105,8 @@ struct Ctx {
     const double *sigA, *sigS, *fleck, *rwSigT;
     const uint8_t *rwElig;
     double *eint, *eradAvg;
-    double *att;             // per cell: attenuation not yet added to the two tallies (gray problems; zero between steps)
+    double *att;             // per cell: attenuation not yet added to the two tallies (gray problems; zero from the
+                             // prestep to the transport, and after the fold)
     uint32_t *segs;
     RwTables rw;
     int32_t *err;            // [0] code, [1] cell lo, [2] particle lo

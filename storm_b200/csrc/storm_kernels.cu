@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(PRESTEP_THREADS, MG ? 4 : 1) k_prestep(Ctx C, 
         A.sigA[c] = sa;
         A.sigS[c] = ss;
         A.eradAvg[c] = 0.0;
+        if (!MG && C.att) C.att[c] = 0.0;   // a step that failed between transport and fold leaves sums here
         double cv;
         if (M.eosKind == STORM_EOS_LINEAR) {
             cv = M.cvPerMass;
