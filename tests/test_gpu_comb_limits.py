@@ -105,3 +105,19 @@ def test_weights_too_small_to_split_are_kept(kind, nx):
         hot = post.weight[post.cell == 11]
         assert len(hot) >= 50 and abs(hot.sum() - 1.75) < 1e-12 and (hot > 0).all()
         assert post.n == 3 + len(hot)
+
+
+@pytest.mark.parametrize("copies", [31, 32, 33, 255, 256, 257, 5000])
+@pytest.mark.parametrize("n", [1, 12, 300, 2500])
+def test_many_copies(oracle_lib, n, copies):
+    """Particles alone in their cells, and some beside others, split into few and many
+    copies; the second comb writes into banks that the first one has grown."""
+    if n * copies > 2_000_000:
+        copies //= 10
+    p = problems.gray_slab(nx=n, new_photons_per_cell=1, face_packets=10, comb_nmin=copies, comb_factor=0.5)
+    cell = np.concatenate([np.arange(n), np.repeat(np.arange(0, n, 3), 5)]).astype(np.uint32)
+    weight = np.concatenate([np.ones(n), 0.01 * np.ones(len(cell) - n)])
+    e = Engine(p)
+    pre = census(p, cell, weight)
+    e.population_control(pre)
+    same_as_oracle(oracle_lib, p, e, pre)
