@@ -1125,7 +1125,9 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
     ALLOC(h->chunkCounts, 32);
     ALLOC(A.level, N);
     ZERO(A.level, N);
-    if (d->groups < 2 && !d->with_hydro) {
+    // the transports that tally by stays (SegmentTallyRun): the gray ones at rest, but
+    // not with reproducible tallies, nor the FP64 DDMC form, which is multigroup's too
+    if (d->groups < 2 && !d->with_hydro && !d->reproducible_tallies && (h->fp32 || poly || !d->with_ddmc)) {
         ALLOC(h->att, N);
         ZERO(h->att, N * sizeof(double));
     }
