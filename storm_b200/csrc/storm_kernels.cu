@@ -1463,7 +1463,7 @@ struct Form64T {
                                                  uint32_t draw) {
         census_store64(b, q, t.p, pid, draw);
     }
-    template <bool LATER, bool JUMPS, class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
         PhysOut o = physics_step<V, LATER>(C, t, rng, tal);
         if (o.errCode) { err = o.errCode; return OUT_ERROR; }
@@ -1521,7 +1521,7 @@ struct Form32T {
                                                  uint32_t draw) {
         census_store32(b, q, t, pid, draw);
     }
-    template <bool LATER, bool JUMPS, class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
         int m = segment32<false, LATER, RNG, TALLY, POLY, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
@@ -1564,7 +1564,7 @@ struct Form32MGT {
                                                  uint32_t draw) {
         census_store32_mg(b, q, t, pid, draw);
     }
-    template <bool LATER, bool JUMPS, class RNG, class TALLY>
+    template <bool LATER, class RNG, class TALLY>
     static __device__ __forceinline__ int seg(const Ctx &C, T &t, RNG &rng, TALLY &tal, int &usedRW, int &err) {
         int m = segment32<true, LATER, RNG, TALLY, false, DDMC>(C, t, rng, tal, usedRW, err);
         if (m == OUT_ERROR && !err) err = STORM_DERR_NOT_ON_BOUNDARY;
@@ -1612,7 +1612,7 @@ __device__ __forceinline__ void visit_bank(const Ctx &C, const Bank &in, uint32_
                 tal.enter(cell0);
                 ++s;
                 int usedRW = 0, err = 0;
-                outcome = F::template seg<false, false>(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
                 rw += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
@@ -1797,7 +1797,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                     tal.enter(cell0);
                     ++segsThis;
                     int usedRW = 0, err = 0;
-                    outcome = F::template seg<true, F::kJumpsLater>(C, t, rng, tal, usedRW, err);
+                    outcome = F::template seg<true>(C, t, rng, tal, usedRW, err);
                     rws += usedRW;
                     if (outcome == OUT_SCATTER || outcome == OUT_REEMIT) {
                         left = outcome;
@@ -1825,7 +1825,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport_refill(Ctx C, Bank in, 
                 tal.enter(cell0);
                 ++segsThis;
                 int usedRW = 0, err = 0;
-                outcome = F::template seg<false, F::kJumpsLater>(C, t, rng, tal, usedRW, err);
+                outcome = F::template seg<false>(C, t, rng, tal, usedRW, err);
                 rws += usedRW;
                 if (outcome != OUT_CONTINUE) {
                     if (outcome == OUT_ERROR) raise_error(C, err, cell0, pid);
