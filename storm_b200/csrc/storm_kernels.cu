@@ -2157,7 +2157,13 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint64_t *kin, 
 // and the caller falls back to the radix sort.
 
 constexpr uint32_t BUCKET_WARP_MAX = 512;     // runs up to this length: one warp (registers to 128, then 4 KB of shared memory)
-constexpr uint32_t BUCKET_WARP_FEW = 128;     // the same where there are too few runs to fill the chip with warps
+constexpr uint32_t BUCKET_WARP_FEW = 128;     // the same for at most BUCKET_FEW_RUNS runs
+// A block of 1024 sorts a run of 129 to 512 keys in about 9 us, a warp in 25 (150
+// keys) to 58 us (400), but the warps' runs go side by side: three runs a
+// multiprocessor are the blocks' part (150 keys, blocks and warps: 100 runs 8.4 and
+// 25 us, 1000 runs 46 and 26, 4000 runs 177 and 39; 400 keys: 10 and 57, 60 and 59,
+// 239 and 93).
+constexpr uint32_t BUCKET_FEW_RUNS = 3 * 148;
 constexpr uint32_t BUCKET_BLOCK_MAX = 8192;   // longer runs up to this length: one block, 64 KB
 constexpr int BUCKET_WARPS = 8;
 constexpr uint32_t BUCKET_LONG_THREADS = 1024;
@@ -3803,7 +3809,7 @@ void launch_bucket_sort(cudaStream_t s, const Ctx &C, const CensusBank &cen, con
     k_bucket_place<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(keys, n, pidBits, nRuns, cursor, outKeys, outVals);
     k_bucket_sort_runs<<<grid_for(nRuns, BUCKET_WARPS, 148 * 32), 32 * BUCKET_WARPS, 0, s>>>(
         C, cen, wc, outKeys, outVals, wS, start, nRuns, pidBits, longRuns, flags, longCap,
-        nRuns < 4096u ? BUCKET_WARP_FEW : BUCKET_WARP_MAX);
+        nRuns <= BUCKET_FEW_RUNS ? BUCKET_WARP_FEW : BUCKET_WARP_MAX);
     const size_t smem = sizeof(uint64_t) * BUCKET_BLOCK_MAX;
     cudaFuncSetAttribute(k_bucket_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     k_bucket_sort_long<<<148, BUCKET_LONG_THREADS, smem, s>>>(C, cen, wc, outKeys, outVals, wS, start, pidBits, longRuns, flags,

@@ -121,3 +121,12 @@ def test_many_copies(oracle_lib, n, copies):
     pre = census(p, cell, weight)
     e.population_control(pre)
     same_as_oracle(oracle_lib, p, e, pre)
+
+
+@pytest.mark.parametrize("nx", [148, 444, 445, 2000])
+def test_run_lengths_either_side_of_the_block_sort(oracle_lib, nx):
+    """Runs of 129 to 512 keys: by blocks where there are few runs, else by warps."""
+    p = problems.gray_slab(nx=nx, new_photons_per_cell=1, face_packets=10, comb_nmin=100, comb_factor=1.5)
+    rng = np.random.default_rng(nx)
+    cell = np.repeat(rng.permutation(nx)[:140], np.tile((1, 127, 128, 129, 255, 256, 257, 400, 511, 512, 513, 600, 64, 33), 10))
+    same_as_oracle(oracle_lib, p, Engine(p), census(p, cell, np.exp(rng.standard_normal(len(cell)))))
