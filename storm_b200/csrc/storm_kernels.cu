@@ -3153,38 +3153,30 @@ __global__ void k_comb_emit(Ctx C, CensusBank cen, const uint32_t *idx, const ui
 // source is the sorted particle src[o].  Every lane writes one particle, so
 // the bank writes are contiguous and no lane idles on a dropped particle.
 // src[o] is written by its particle's thread, or, where a particle has more than
-// EMIT_SRC_ALONE copies, by all threads of its block: a particle alone in its cell
+// EMIT_SRC_ALONE copies, by all lanes of its warp: a particle alone in its cell
 // can have thousands (100 such particles of 1e4 copies each: the comb's call 0.82 to
 // 0.18 ms; with marks and a running maximum over the slots, whatever the copies, 0.24).
-// A block takes `per` particles at a time, fewer where there are too few to fill the chip.
+// A warp takes `per` particles at a time, fewer than 32 where there are too few to
+// fill the chip.
 constexpr uint32_t EMIT_SRC_ALONE = 32;
-constexpr uint32_t EMIT_SRC_THREADS = 256;
-__global__ void __launch_bounds__(EMIT_SRC_THREADS) k_emit_src(Ctx C, const uint64_t *sortedKeys, int pidBits,
-                                                               uint32_t bins, const uint32_t *pCount,
-                                                               const uint32_t *pOff, const uint64_t *groupOff,
-                                                               uint32_t nValid, uint32_t per, uint32_t *src) {
-    __shared__ uint64_t at[EMIT_SRC_THREADS];
-    __shared__ uint32_t copies[EMIT_SRC_THREADS], from[EMIT_SRC_THREADS], many;
-    for (uint32_t base = blockIdx.x * per; base < nValid; base += gridDim.x * per) {
-        if (threadIdx.x == 0) many = 0;
-        __syncthreads();
-        const uint32_t q = base + threadIdx.x;
-        const uint32_t n = threadIdx.x < per && q < nValid ? pCount[q] & ~KEEP : 0u;
-        if (n) {
-            const uint64_t o = first_copy(C, sortedKeys[q] >> pidBits, bins, groupOff, pOff[q]);
-            if (n <= EMIT_SRC_ALONE) {
-                for (uint32_t k = 0; k < n; ++k) src[o + k] = q;
-            } else {
-                const uint32_t e = atomicAdd(&many, 1u);
-                at[e] = o;
-                copies[e] = n;
-                from[e] = q;
-            }
+__global__ void __launch_bounds__(256) k_emit_src(Ctx C, const uint64_t *sortedKeys, int pidBits, uint32_t bins,
+                                                  const uint32_t *pCount, const uint32_t *pOff, const uint64_t *groupOff,
+                                                  uint32_t nValid, uint32_t per, uint32_t *src) {
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x / 32);
+    const uint64_t stride = static_cast<uint64_t>(warps) * per;
+    for (uint64_t base = static_cast<uint64_t>(blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * per; base < nValid;
+         base += stride) {
+        const uint32_t q = static_cast<uint32_t>(base) + lane;
+        const uint32_t n = lane < per && base + lane < nValid ? pCount[q] & ~KEEP : 0u;
+        const uint64_t o = n ? first_copy(C, sortedKeys[q] >> pidBits, bins, groupOff, pOff[q]) : 0u;
+        if (n <= EMIT_SRC_ALONE)
+            for (uint32_t k = 0; k < n; ++k) src[o + k] = q;
+        for (unsigned many = __ballot_sync(FULL, n > EMIT_SRC_ALONE); many; many &= many - 1) {
+            const int l = __ffs(many) - 1;
+            const uint32_t nl = __shfl_sync(FULL, n, l), ql = __shfl_sync(FULL, q, l);
+            uint32_t *to = src + __shfl_sync(FULL, o, l);
+            for (uint32_t k = lane; k < nl; k += 32) to[k] = ql;
         }
-        __syncthreads();
-        for (uint32_t e = 0; e < many; ++e)
-            for (uint32_t k = threadIdx.x; k < copies[e]; k += EMIT_SRC_THREADS) src[at[e] + k] = from[e];
-        __syncthreads();
     }
 }
 
@@ -3872,9 +3864,9 @@ void launch_comb_emit_out(cudaStream_t s, const Ctx &C, const CensusBank &cen, c
                           const uint32_t *pCount, const double *pWeight, const uint32_t *pOff, const uint64_t *groupOff,
                           uint32_t *src, const Bank &out) {
     if (!nValid || !total) return;
-    const uint32_t per = std::min(std::max(nValid / (148u * 8u), 1u), EMIT_SRC_THREADS);
-    k_emit_src<<<grid_for(nValid, per, 148 * 16), EMIT_SRC_THREADS, 0, s>>>(C, sortedKeys, pidBits, bins, pCount, pOff,
-                                                                            groupOff, nValid, per, src);
+    const uint32_t per = std::min(std::max(nValid / (148u * 64u), 1u), 32u);
+    k_emit_src<<<grid_for(nValid, 8 * per, 148 * 16), 256, 0, s>>>(C, sortedKeys, pidBits, bins, pCount, pOff, groupOff,
+                                                                   nValid, per, src);
     if (C.fp32)
         k_comb_emit_out<true><<<grid_for(total, 256, 148 * 16), 256, 0, s>>>(C, cen, idx, sortedKeys, pidBits, bins, total,
                                                                              src, pCount, pWeight, out);
