@@ -2747,19 +2747,20 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_comb_plan(Ctx C, CombParams
                                                                uint32_t *pCount, double *pWeight, uint32_t *pOff,
                                                                uint64_t *cellCount, double *eradCensus, DevStats *st,
                                                                const uint32_t *unsorted, uint32_t batch) {
-    if (unsorted && *unsorted) return;
     constexpr uint32_t COPIES = 256;   // copies of 32 particles that are laid out for the chain
     __shared__ __align__(16) double stage[WALK_WARPS][COPIES + 8];
+    const uint32_t skip = unsorted ? *unsorted : 0u;   // on its way with the loads below
     const double tot = *Wtot;
-    if (!isfinite(tot)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
-    }
-    const bool none = tot == 0.0 || !isfinite(tot);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double *x = stage[wid];
     const uint32_t c = (blockIdx.x * WALK_WARPS + wid) * batch + lane;
     const bool mine = lane < batch && c < C.ncells;
     const uint32_t a = mine ? start[c] : 0u, b = mine ? start[c + 1] : 0u;
+    if (skip) return;
+    if (!isfinite(tot)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(C, STORM_DERR_COMB_TOTAL, 0, 0);
+    }
+    const bool none = tot == 0.0 || !isfinite(tot);
     CombCell cc{};
     double Wc = 0.0;
     if (b > a && !none) {
