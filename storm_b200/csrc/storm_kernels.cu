@@ -1489,6 +1489,9 @@ struct Form64T {
     static __device__ __forceinline__ double weight(const T &t) { return t.p.w; }
 };
 using Form64 = Form64T<0, SegmentTallyRun>;
+// Multigroup with DDMC, and gray DDMC on the Cartesian grid, which has no form of its
+// own: it tallies per segment, takes its jumps inside the burst and runs three blocks
+// a multiprocessor, as multigroup does.
 using Form64Full = Form64T<1>;
 using Form64Poly = Form64T<2, SegmentTallyRun>;
 using Form64PolyDDMC = Form64T<5, SegmentTallyRun>;   // Form64Poly with the DDMC branch
@@ -1546,7 +1549,7 @@ using Form32PolyDDMCFix = Form32T<true, true, SegmentTallyFixed>;
 template <bool DDMC = true, class TL = SegmentTally>
 struct Form32MGT {
     static constexpr bool kTogether = true;
-    static constexpr bool kJumpsLater = false;   // every other segment is a jump
+    static constexpr bool kJumpsLater = false;   // as in FP32 gray; not measured
     using T = Track32;
     using Rng = PhiloxRng4;      // bank visits
     using Ring = PhiloxRing4;    // the persistent transport
@@ -1678,14 +1681,16 @@ __global__ void __launch_bounds__(256, MINB) k_transport32(Ctx C, Bank in, const
 // or instruction fetch and divergence (FP64, multigroup), dependent loads of the
 // face planes on polyhedral meshes; a problem of few cells or few, long
 // histories by the chain of its longest history.
-// Transport of the second step, before and after the rings, the run tally, the
-// finish and the leaner refill: 64^3 gray cube, 4.2e8 segments, FP32 7.5 to 5.8 ms,
-// FP64 19.6 to 18.3; 24^3, 2.1e7 segments, FP32 0.78 to 0.50; 100-cell slab, 8e6
-// segments, FP64 3.1 to 1.4; 72^3 x 64 groups, 2.6e7 segments, FP32 2.77 to 1.90;
-// Voronoi 4e4 cells, 8.6e7 segments, FP32 6.4 to 6.2.
+// Transport of the second step before the rings, the run tally, the finish, the
+// leaner refill and what followed them, and now: 64^3 gray cube, 4.4e8 segments,
+// FP32 7.5 and 5.7 ms, FP64 19.6 and 13.9; 24^3, 1.9e7 segments, FP32 0.78 and 0.44;
+// 100-cell slab, 7.9e6 segments, FP64 3.1 and 1.4; 72^3 x 64 groups, 2.6e7 segments,
+// FP32 2.77 and 1.75; Voronoi 4e4 cells, 8.5e7 segments, FP32 6.4 and 5.4.
 // A step of few histories ends with its longest one, so long ones are to start
-// first: the chunks are taken in the order of their cells' expected events
-// (history_level), cell order within a level.
+// first: the chunks are taken by level, the highest first and in no order within a
+// level.  A chunk's level is the expected events (history_level) in the cell of its
+// first or of its last particle, whichever are more; the cells between are not
+// looked at.
 constexpr int LEVELS = 16;
 __global__ void k_chunk_levels(const uint32_t *cell, const uint8_t *level, uint32_t n, uint32_t chunk, uint32_t nChunks,
                                uint8_t *chunkLevel, uint32_t *count) {
@@ -2515,7 +2520,7 @@ __global__ void k_sorted_weights(Ctx C, CensusBank cen, const uint32_t *idx, uin
 // The comb's walks along a run add FP64 weights left to right, so that every sum
 // rounds as the reference's: a serial chain per run.  k_comb_cell_sums is the one
 // kernel that walks all of it, and it leaves the running weight at each particle
-// for the plan.  A warp takes `batch` neighbouring runs (up to 32 where there are
+// for the plan.  A warp takes `batch` neighbouring runs (up to 8 where there are
 // more runs than warps on the chip) and goes over their particles, which are
 // contiguous, in tiles: the tile is loaded coalesced into shared memory, the next
 // one on its way, and each lane walks its own run's part of it there.  So a long

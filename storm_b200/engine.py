@@ -318,6 +318,9 @@ class Engine:
         return out
 
     def cells(self):
+        """The cell arrays, by name.  On meshes below 524288 cells they are parts of one
+        allocation, which lives as long as any of them: copy an array to keep it
+        without the others (or take temperature())."""
         keys = ("temperature", "internal_energy", "erad_time_avg", "erad_census", "sigma_a", "fleck")
         # Every element is written by the call.  Arrays below 4 MB, for which numpy asks
         # for no huge pages, are parts of one allocation: as seven fresh ones they are
