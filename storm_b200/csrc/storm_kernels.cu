@@ -997,6 +997,17 @@ __device__ inline void sample_in_poly_cell(const Ctx &C, uint32_t cell, RNG &rng
     pz = a0 * C.vtx[3 * v0 + 2] + a1 * C.vtx[3 * v1 + 2] + a2 * C.vtx[3 * v2 + 2] + a3 * cz;
 }
 
+// Ctx::cfX32, the FP32 form's crossing table (a ghost has no mesh point).  Made here
+// since the host's loop over the slots and its upload took 3 of the 40 ms of a
+// handle's creation (4e4 cells).
+__global__ void k_poly_cross(Ctx C, float4 *cross) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < C.ncells; c += gridDim.x * blockDim.x)
+        for (uint32_t q = C.cfo[c]; q < C.cfo[c + 1]; ++q) {
+            const uint32_t nb = C.cfNext[q], at = nb < C.ncells ? nb : c;
+            cross[q] = make_float4(static_cast<float>(C.mpx[c] - C.mpx[at]), static_cast<float>(C.mpy[c] - C.mpy[at]),
+                                   static_cast<float>(C.mpz[c] - C.mpz[at]), __uint_as_float(nb));
+        }
+}
 // The table sample_in_poly_cell looks up: per cell its fan tetrahedra in the
 // sampler's order, each with the running sum of the volumes up to it, formed by
 // the sampler's own operations in its order (so equal to its sums bit for bit),
@@ -3691,6 +3702,9 @@ void launch_emit_cells(cudaStream_t s, const Ctx &C, const CellArrays &A, const 
 }
 __global__ void k_set_u32(uint32_t *p, uint32_t v) { *p = v; }
 void launch_set_u32(cudaStream_t s, uint32_t *p, uint32_t v) { k_set_u32<<<1, 1, 0, s>>>(p, v); }
+void launch_poly_cross(cudaStream_t s, const Ctx &C, float4 *cross) {
+    k_poly_cross<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, cross);
+}
 void launch_poly_tets(cudaStream_t s, const Ctx &C, const uint32_t *tetOff, double *tetCum, uint2 *tetAT) {
     k_poly_tets<<<grid_for(C.ncells, 128, 8192), 128, 0, s>>>(C, tetOff, tetCum, tetAT);
 }

@@ -1103,17 +1103,7 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
                 }
             ALLOC(h->cfN32, K);
             H2D(h->cfN32, pl.data(), K);
-            std::vector<float4> cross(K);
-            for (uint32_t c = 0; c < N; ++c)
-                for (uint32_t q = mesh->cell_face_offset[c]; q < mesh->cell_face_offset[c + 1]; ++q) {
-                    const uint32_t nb = nextv[q], at = nb < N ? nb : c;   // a ghost has no mesh point
-                    float bits;
-                    std::memcpy(&bits, &nb, sizeof(bits));
-                    cross[q] = make_float4(static_cast<float>(mp[0][c] - mp[0][at]), static_cast<float>(mp[1][c] - mp[1][at]),
-                                           static_cast<float>(mp[2][c] - mp[2][at]), bits);
-                }
-            ALLOC(h->cfX32, K);
-            H2D(h->cfX32, cross.data(), K);
+            ALLOC(h->cfX32, K);   // made on the device (launch_poly_cross)
         }
     }
     H2D(A.T, d->temperature, N);
@@ -1212,6 +1202,10 @@ int storm_cuda_create(const StormProblemDesc *d, StormHandle **out) {
         C.poly = 1;
         C.cfo = h->cfo; C.cfN = h->cfN; C.cfP = h->cfP; C.cfNext = h->cfNext; C.cfFace = h->cfFace; C.cfA = h->cfA;
         C.mpx = h->mpx; C.mpy = h->mpy; C.mpz = h->mpz;
+        if (h->cfX32) {
+            launch_poly_cross(h->stream, C, h->cfX32);
+            if (cudaGetLastError() != cudaSuccess) return fail(STORM_ERR_CUDA);
+        }
         C.fvo = h->fvo; C.fvi = h->fvi; C.vtx = h->vtx; C.chord = h->chord; C.cfN32 = h->cfN32; C.cfX32 = h->cfX32;
         if (h->tetCum) {
             launch_poly_tets(h->stream, C, h->tetOff, h->tetCum, h->tetAT);
