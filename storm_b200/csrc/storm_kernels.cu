@@ -2174,12 +2174,12 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint64_t *kin, 
 
 constexpr uint32_t BUCKET_WARP_MAX = 512;     // runs up to this length: one warp (registers to 128, then 4 KB of shared memory)
 constexpr uint32_t BUCKET_WARP_FEW = 128;     // the same for at most BUCKET_FEW_RUNS runs
-// A block of 1024 sorts a run of 129 to 512 keys in about 9 us, a warp in 25 (150
-// keys) to 58 us (400), but the warps' runs go side by side: three runs a
-// multiprocessor are the blocks' part (150 keys, blocks and warps: 100 runs 8.4 and
-// 25 us, 1000 runs 46 and 26, 4000 runs 177 and 39; 400 keys: 10 and 57, 60 and 59,
-// 239 and 93).
-constexpr uint32_t BUCKET_FEW_RUNS = 3 * 148;
+// A block of 1024 sorts a run of 129 to 512 keys in 7 to 9 us, a warp in 25 (to 256
+// keys) or 58, but the warps' runs go side by side: up to four runs a multiprocessor
+// are the blocks' part (runs of 150 keys, blocks and warps: 100 runs 8.4 and 25 us,
+// 592 runs 29.8 and 27.3, 1000 runs 46 and 26, 4000 runs 177 and 39; of 400 keys: 10
+// and 57, 37.6 and 59.4, 60 and 59, 239 and 93).
+constexpr uint32_t BUCKET_FEW_RUNS = 4 * 148;
 constexpr uint32_t BUCKET_BLOCK_MAX = 8192;   // longer runs up to this length: one block, 64 KB
 constexpr int BUCKET_WARPS = 8;
 constexpr uint32_t BUCKET_LONG_THREADS = 1024;

@@ -123,7 +123,7 @@ def test_many_copies(oracle_lib, n, copies):
     same_as_oracle(oracle_lib, p, e, pre)
 
 
-@pytest.mark.parametrize("nx", [148, 444, 445, 2000])
+@pytest.mark.parametrize("nx", [148, 592, 593, 2000])
 def test_run_lengths_either_side_of_the_block_sort(oracle_lib, nx):
     """Runs of 129 to 512 keys: by blocks where there are few runs, else by warps."""
     p = problems.gray_slab(nx=nx, new_photons_per_cell=1, face_packets=10, comb_nmin=100, comb_factor=1.5)
