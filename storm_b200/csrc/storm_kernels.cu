@@ -2546,9 +2546,12 @@ static inline uint32_t walk_batch(uint32_t nRuns) {
     return b < 1 ? 1u : (b > 8 ? 8u : b);
 }
 // A thread per run where there are runs enough to fill the chip and most are empty
-// or single (72^3 cells, 2e4 particles: sums 4.7 us and plan 15 us, by warps 14 and 63);
-// with 50 particles a run the warps are ahead (64^3 cells: sums 84 and plan 180 us, by
-// threads 38 and 421).
+// or single (72^3 cells, 2e4 particles: sums 3.4 us and plan 13 us, by warps 14 and 63);
+// with 50 particles a run the warps are ahead (64^3 cells: sums 64 and plan 186 us, by
+// threads 38 and 421).  Evenly short runs would take threads from 3e4 cells and up to
+// 8 particles on (99000 cells of 3: plan 10 us, by warps 41; 3e5 of 5: 31 and 107), but
+// a thread walks a crowded run among them at about 1 us a particle, and the average
+// says nothing of it.
 static inline bool walk_by_thread(uint32_t n, uint32_t nRuns) { return nRuns >= 100000u && n / nRuns < 4u; }
 static inline uint32_t walk_grid(uint32_t nRuns) {
     const uint32_t perBlock = WALK_WARPS * walk_batch(nRuns);
@@ -2628,9 +2631,10 @@ __global__ void k_comb_cell_sums_thread(const double *wS, const uint32_t *start,
 // Deterministic total: partial sum t adds v[t], v[t + 1024], ... in order
 // (coalesced), then a pairwise tree over the 1024 partial sums.  Above
 // SUM_ONE_BLOCK values the partial sums are spread over SUM_BLOCKS blocks and the
-// last one to finish takes the tree (one block reads 2 MB in 22 us at 64^3 cells);
+// last one to finish takes the tree (one block and several: 30000 values 4.5 and 6.9
+// us, 64000 6.8 and 8.3, 99000 7.5 and 8.3, 64^3 22 and 13.8);
 // scratch: 1024 partial sums and a counter, zero before and after.
-constexpr uint32_t SUM_ONE_BLOCK = 16384, SUM_BLOCKS = 32;
+constexpr uint32_t SUM_ONE_BLOCK = 131072, SUM_BLOCKS = 32;
 __device__ __forceinline__ double strided_sum(const double *v, uint32_t n, uint32_t t) {
     double s = 0.0;
     uint32_t q = t;

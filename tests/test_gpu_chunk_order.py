@@ -74,9 +74,9 @@ def test_histories_do_not_depend_on_the_chunks_order(oracle_lib, bank, ordered, 
             np.testing.assert_array_equal(getattr(got, k), getattr(want, k), err_msg=k)
 
 
-@pytest.mark.parametrize("nx", [1023, 16384, 16385, 17407, 32769, 65536])
+@pytest.mark.parametrize("nx", [1023, 16385, 131072, 131073, 132095, 163841])
 def test_total_weight(oracle_lib, nx):
-    """The total that every cell's share is taken of: by one block up to 16384 cells, by
+    """The total that every cell's share is taken of: by one block up to 131072 cells, by
     several above, the same partial sums; the first and the last cells weigh most."""
     p = problems.gray_slab(nx=nx, new_photons_per_cell=1, face_packets=10, comb_nmin=2, comb_factor=3.0)
     rng = np.random.default_rng(nx)
